@@ -3,11 +3,26 @@
 //
 // vt-transformer sends its 32-bit products to cuBLASLt and lets it pick tensor operations
 // (v1/tensortype/cuda_kernels/lt_sgemm.cu:53-54), so it has no verified 32-bit run.  With float
-// operands this kernel is the engine's 32-bit path: every output element is the sum, over the
+// operands these kernels are the engine's 32-bit path: every output element is the sum, over the
 // runs of 16 consecutive k in their order, of each run's sum over its k in their order (two
-// levels: the rounding error grows with 16 + K / 16 terms, not with K), whatever M is and whatever
-// else is in the batch, so logits agree bit for bit however the tokens are cut into steps.  With bfloat16 operands it is the
-// plain twin of the tensor-core products.
+// levels: the rounding error grows with 16 + K / 16 terms, not with K), whatever M is, whichever kernel
+// runs and whatever else is in the batch, so logits agree bit for bit however the tokens are cut into
+// steps.  With bfloat16 operands they are the plain twin of the tensor-core products.
+//
+// Two kernels that form the same sums in the same order:
+//
+// * gemm_stream_kernel, few rows of A.  Bound by the bytes of W, each read once.  A warp owns F rows of W and goes
+//   along K in chunks of 32 runs, a lane a run: the chunk comes into shared memory with cp.async through a ring (the
+//   chunk of A once for the CTA's warps), a lane takes its run of W and of each row of A into registers and forms a chain
+//   of 16 multiply-adds, and the lanes' sums meet in shared memory again, where one lane an output adds them in the
+//   order of the runs.  A CTA walks several groups of rows without letting its ring run dry.
+// * gemm_tile_kernel, many rows.  Bound by what shared memory delivers to the FMA pipe: a tile of 64 x 64 outputs a CTA of 64 threads,
+//   8 x 8 outputs a thread, takes 16 numbers for 64 multiply-adds a k; the next 16 k are on their way in registers meanwhile.
+//   Where such tiles are fewer than the SMs, tiles of 32 x 32 by 4 x 4 outputs a thread keep more of them busy.
+//
+// Measured on a B200, us, before (one kernel, tiles of 64 x 64 by 256 threads) and now: 3 rows by 1152 x 896: 71 and 10, by 896 x 4864:
+// 358 and 17, by 151936 x 896: 537 and 195; 388 rows by 1152 x 896: 66 and 62, by 9728 x 896: 268 and 244, by 896 x 4864: 330 and 251;
+// 1,024 rows by 4608 x 3584: 1,057 and 936 (36 TFLOP/s).  Packed multiply-adds (fma.rn.f32x2) and tiles of 128 x 128 were level.
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.cuh"
@@ -15,8 +30,27 @@
 namespace vtb {
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, PAD = 4;
+constexpr int kRun = 16;              // consecutive k whose products are one chain
+constexpr int kChunk = 32 * kRun;     // of the streaming kernel: a run a lane
+constexpr int kStreamWarps = 8;
+
+// Rows of A that the streaming kernel takes, where a warp has one row of W (it reads W once for every 8 of them) and where it has
+// several; and the rows of W from which it does (fewer leave SMs without warps).  At 64 rows by 896 x 4864 it takes 104 us and the tiles 215,
+// at 128 rows 188 and 207; by 151936 x 896 at 8 rows 367 and 539, at 16 rows 711 and 539.
+constexpr int kStreamRows = 64, kStreamRowsWide = 8;
+constexpr int kStreamFourRows = 4 * kStreamWarps * 148;
+
+// A run in shared memory: its 16 numbers and 16 bytes that keep eight lanes' loads apart.
+template <typename T> __host__ __device__ constexpr int run_bytes() { return kRun * (int)sizeof(T) + 16; }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool in) {
+    const int n = in ? 16 : 0;                            // (nothing is read and 16 zeros are written if not)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+}  // namespace
 
 template <typename T> __device__ __forceinline__ float4 load4(const T* p);
 template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -27,74 +61,256 @@ template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bf
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
-template <typename TA, typename TC>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const TA* __restrict__ a, const TA* __restrict__ w, const float* __restrict__ bias,
-                 TC* __restrict__ c, int m, int n, int k) {
+// The 16 numbers of a run in shared memory.
+template <typename T> __device__ __forceinline__ void load_run(const unsigned char* p, float (&v)[kRun]) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 t = *reinterpret_cast<const float4*>(p + 16 * q);
+            v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            float t[8];
+            Vec8<__nv_bfloat16>::load(reinterpret_cast<const __nv_bfloat16*>(p + 16 * q), t);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[8 * q + e] = t[e];
+        }
+    }
+}
+
+// F rows of W a warp, MT rows of A (blockIdx.y the group of them), a ring of STAGES chunks.
+template <typename T, int MT, int F, int STAGES> __host__ __device__ constexpr int stream_smem() {
+    return STAGES * 32 * run_bytes<T>() * (kStreamWarps * F + MT) + kStreamWarps * MT * F * 36 * 4;
+}
+
+template <typename TA, typename TC, int MT, int F, int STAGES>
+__global__ void __launch_bounds__(32 * kStreamWarps)
+gemm_stream_kernel(const TA* __restrict__ a, const TA* __restrict__ w, const float* __restrict__ bias, TC* __restrict__ c, int m,
+                   int n, int k) {
+    static_assert(MT * F <= 32, "a lane an output");
+    constexpr int kRunBytes = run_bytes<TA>(), kRowBytes = 32 * kRunBytes, kPieces = kRun * (int)sizeof(TA) / 16;
+    constexpr int kStage = kRowBytes * (kStreamWarps * F + MT), kPiece = 16 / (int)sizeof(TA);      // (numbers in 16 bytes)
+    extern __shared__ __align__(16) unsigned char ring[];
     pdl_launch();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m0 = blockIdx.y * MT;
+    const int chunks = (k + kChunk - 1) / kChunk;
+    // the CTA's groups of kStreamWarps * F rows of W, one after the other: chunk s of the CTA is chunk s % chunks of its group s / chunks
+    const int groups = (n + kStreamWarps * F - 1) / (kStreamWarps * F), mine = (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int steps = mine * chunks;
+    float* sums = reinterpret_cast<float*>(ring + STAGES * kStage) + warp * (MT * F * 36);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(ring);
+    // a row's chunk: pieces of 16 bytes, a warp's lanes side by side; piece i of a run lies at run * kRunBytes + 16 i
+    auto fetch_row = [&](const TA* row, uint32_t dst, int chunk, bool in) {
+#pragma unroll
+        for (int q = 0; q < kPieces; ++q) {
+            const int piece = q * 32 + lane, at = chunk * kChunk + piece * kPiece;
+            const bool ok = in && at < k;                 // (k is a multiple of 8 numbers: a piece is inside or outside whole)
+            cp_async16(dst + piece / kPieces * kRunBytes + piece % kPieces * 16, ok ? row + at : row, ok);
+        }
+    };
+    auto fetch_w = [&](int s) {
+        const uint32_t dst = base + s % STAGES * kStage + warp * F * kRowBytes;
+        const int n0 = (((int)blockIdx.x + s / chunks * (int)gridDim.x) * kStreamWarps + warp) * F;
+#pragma unroll
+        for (int f = 0; f < F; ++f) fetch_row(w + (size_t)min(n0 + f, n - 1) * k, dst + f * kRowBytes, s % chunks, s < steps && n0 + f < n);
+    };
+    auto fetch_a = [&](int s) {
+        const uint32_t dst = base + s % STAGES * kStage + kStreamWarps * F * kRowBytes;
+        for (int i = warp; i < MT; i += kStreamWarps) fetch_row(a + (size_t)min(m0 + i, m - 1) * k, dst + i * kRowBytes, s % chunks, s < steps && m0 + i < m);
+    };
+    // (the weights are no kernel's result: they may be sent for before the kernels in front have ended)
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) fetch_w(s);
     pdl_wait();
-    __shared__ __align__(16) float as[BK][BM + PAD];
-    __shared__ __align__(16) float ws[BK][BN + PAD];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int lrow = tid >> 2, lk = (tid & 3) * 4;   // loader: row of the tile, 4 consecutive k
-    const int ty = tid >> 4, tx = tid & 15;          // compute: rows ty*4.., cols tx*4..
-    float acc[4][4] = {};
-
-    const bool a_ok = (m0 + lrow) < m, w_ok = (n0 + lrow) < n;
-    const TA* ap = a + (size_t)(m0 + lrow) * k + lk;
-    const TA* wp = w + (size_t)(n0 + lrow) * k + lk;
-
-    for (int k0 = 0; k0 < k; k0 += BK) {
-        float4 av = make_float4(0.f, 0.f, 0.f, 0.f), wv = av;
-        if (k0 + lk < k) {   // k % 4 == 0, so the four elements are inside or outside together
-            if (a_ok) av = load4<TA>(ap + k0);
-            if (w_ok) wv = load4<TA>(wp + k0);
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        fetch_a(s);
+        cp_async_commit();
+    }
+    float acc = 0.f;                                      // lane f * MT + i: the output of row i of A and row f of W
+    for (int s = 0; s < steps; ++s) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                                  // this chunk is there, and the slot of the last one is free
+        fetch_w(s + STAGES - 1);                          // (beyond the last: zeros)
+        fetch_a(s + STAGES - 1);
+        cp_async_commit();
+        const unsigned char* at = ring + s % STAGES * kStage + lane * kRunBytes;
+        float wv[F][kRun];
+#pragma unroll
+        for (int f = 0; f < F; ++f) load_run<TA>(at + (warp * F + f) * kRowBytes, wv[f]);
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            float x[kRun], part[F];
+            load_run<TA>(at + (kStreamWarps * F + i) * kRowBytes, x);
+#pragma unroll
+            for (int f = 0; f < F; ++f) part[f] = 0.f;
+#pragma unroll
+            for (int e = 0; e < kRun; ++e)
+#pragma unroll
+                for (int f = 0; f < F; ++f) part[f] = fmaf(x[e], wv[f][e], part[f]);
+#pragma unroll
+            for (int f = 0; f < F; ++f) sums[(f * MT + i) * 36 + lane] = part[f];
         }
-        as[lk + 0][lrow] = av.x; as[lk + 1][lrow] = av.y; as[lk + 2][lrow] = av.z; as[lk + 3][lrow] = av.w;
-        ws[lk + 0][lrow] = wv.x; ws[lk + 1][lrow] = wv.y; ws[lk + 2][lrow] = wv.z; ws[lk + 3][lrow] = wv.w;
-        __syncthreads();
-        float part[4][4] = {};                       // this run of k alone
+        __syncwarp();
+        if (lane < MT * F) {
+            float4 p[8];
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            const float4 x = *reinterpret_cast<const float4*>(&as[kk][ty * 4]);
-            const float4 y = *reinterpret_cast<const float4*>(&ws[kk][tx * 4]);
-            const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+            for (int r = 0; r < 8; ++r) p[r] = *reinterpret_cast<const float4*>(sums + lane * 36 + 4 * r);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int r = 0; r < 8; ++r) {                 // (runs beyond k are zeros)
+                acc += p[r].x;
+                acc += p[r].y;
+                acc += p[r].z;
+                acc += p[r].w;
+            }
+            if (s % chunks == chunks - 1) {
+                const int row = m0 + lane % MT, col = (((int)blockIdx.x + s / chunks * (int)gridDim.x) * kStreamWarps + warp) * F + lane / MT;
+                if (row < m && col < n) c[(size_t)row * n + col] = from_float<TC>(acc + (bias ? bias[col] : 0.f));
+                acc = 0.f;
+            }
+        }
+        __syncwarp();
+    }
+    cp_async_wait<0>();
+}
+
+// B x B outputs a CTA, E x E a thread.
+template <typename TA, typename TC, int B, int E>
+__global__ void __launch_bounds__(64)
+gemm_tile_kernel(const TA* __restrict__ a, const TA* __restrict__ w, const float* __restrict__ bias, TC* __restrict__ c, int m, int n,
+                 int k) {
+    static_assert(B * B == 64 * E * E && E % 4 == 0, "64 threads");
+    constexpr int LOADS = B * kRun / 4 / 64;              // pieces of four k of each tile that a thread fetches
+    constexpr int SIDE = B / E * 4;                       // a thread's rows: 4 ty + 0..3, and the same SIDE further on
+    __shared__ __align__(16) float as[2][kRun][B + 4];    // a k's rows of A side by side
+    __shared__ __align__(16) float ws[2][kRun][B + 4];
+    pdl_launch();
+    const int tid = threadIdx.x, tx = tid % (B / E), ty = tid / (B / E);
+    const int m0 = blockIdx.y * B, n0 = blockIdx.x * B;
+    float4 av[LOADS], wv[LOADS];
+    auto fetch = [&](const TA* from, int first, int rows, int k0, float4 (&v)[LOADS]) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xs[i], ys[j], part[i][j]);
+        for (int i = 0; i < LOADS; ++i) {
+            const int r = first + (tid + 64 * i) % B, at = k0 + (tid + 64 * i) / B * 4;
+            v[i] = (r < rows && at < k) ? load4<TA>(from + (size_t)r * k + at) : make_float4(0.f, 0.f, 0.f, 0.f);      // (k is a multiple of 4)
+        }
+    };
+    auto put = [&](float (&to)[kRun][B + 4], const float4 (&v)[LOADS]) {
+#pragma unroll
+        for (int i = 0; i < LOADS; ++i) {
+            const int r = (tid + 64 * i) % B, at = (tid + 64 * i) / B * 4;
+            to[at][r] = v[i].x;
+            to[at + 1][r] = v[i].y;
+            to[at + 2][r] = v[i].z;
+            to[at + 3][r] = v[i].w;
+        }
+    };
+    float acc[E][E] = {};
+    fetch(w, n0, n, 0, wv);
+    pdl_wait();
+    fetch(a, m0, m, 0, av);
+    put(as[0], av);
+    put(ws[0], wv);
+    __syncthreads();
+    int b = 0;
+    for (int k0 = 0; k0 < k; k0 += kRun, b ^= 1) {
+        const bool more = k0 + kRun < k;
+        if (more) {
+            fetch(w, n0, n, k0 + kRun, wv);
+            fetch(a, m0, m, k0 + kRun, av);
+        }
+        float part[E][E] = {};                            // this run of k alone
+#pragma unroll
+        for (int kk = 0; kk < kRun; ++kk) {
+            float x[E], y[E];
+#pragma unroll
+            for (int i = 0; i < E; i += 4) {
+                const float4 t = *reinterpret_cast<const float4*>(&as[b][kk][i / 4 * SIDE + 4 * ty]);
+                const float4 u = *reinterpret_cast<const float4*>(&ws[b][kk][i / 4 * SIDE + 4 * tx]);
+                x[i] = t.x; x[i + 1] = t.y; x[i + 2] = t.z; x[i + 3] = t.w;
+                y[i] = u.x; y[i + 1] = u.y; y[i + 2] = u.z; y[i + 3] = u.w;
+            }
+#pragma unroll
+            for (int i = 0; i < E; ++i)
+#pragma unroll
+                for (int j = 0; j < E; ++j) part[i][j] = fmaf(x[i], y[j], part[i][j]);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < E; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+            for (int j = 0; j < E; ++j) acc[i][j] += part[i][j];
+        if (more) {
+            put(as[b ^ 1], av);
+            put(ws[b ^ 1], wv);
+        }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int row = m0 + ty * 4 + i;
+    for (int i = 0; i < E; ++i) {
+        const int row = m0 + i / 4 * SIDE + 4 * ty + i % 4;
         if (row >= m) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int col = n0 + tx * 4 + j;
+        for (int j = 0; j < E; ++j) {
+            const int col = n0 + j / 4 * SIDE + 4 * tx + j % 4;
             if (col < n) c[(size_t)row * n + col] = from_float<TC>(acc[i][j] + (bias ? bias[col] : 0.f));
         }
     }
 }
 
+namespace {
+template <typename TA, typename TC, int MT, int F, int STAGES>
+cudaError_t launch_stream_form(const TA* a, const TA* w, const float* bias, TC* c, int m, int n, int k, cudaStream_t stream) {
+    static std::atomic<unsigned long long> done{0};
+    constexpr int smem = stream_smem<TA, MT, F, STAGES>();
+    const cudaError_t e = allow_dynamic_smem(gemm_stream_kernel<TA, TC, MT, F, STAGES>, smem, done);
+    if (e != cudaSuccess) return e;
+    // as many CTAs as the SMs hold at once: each goes on to its next rows without letting its ring run dry
+    const int groups = (n + F * kStreamWarps - 1) / (F * kStreamWarps), resident = 148 * max(1, 227 * 1024 / (smem + 1024));
+    return launch(gemm_stream_kernel<TA, TC, MT, F, STAGES>, dim3(min(groups, resident), (m + MT - 1) / MT), 32 * kStreamWarps, smem, stream, a, w,
+                  bias, c, m, n, k);
+}
+
+template <typename TA, typename TC, int MT>
+cudaError_t launch_stream(const TA* a, const TA* w, const float* bias, TC* c, int m, int n, int k, cudaStream_t stream) {
+    if constexpr (MT == 8) {                              // (two: four would not fit shared memory beside eight rows of A)
+        if (n >= kStreamFourRows) return launch_stream_form<TA, TC, MT, 2, 3>(a, w, bias, c, m, n, k, stream);
+    } else {
+        if (n >= kStreamFourRows) return launch_stream_form<TA, TC, MT, 4, 2>(a, w, bias, c, m, n, k, stream);
+    }
+    return launch_stream_form<TA, TC, MT, 1, 4>(a, w, bias, c, m, n, k, stream);
+}
+
+template <typename TA, typename TC>
+cudaError_t launch_tile(const TA* a, const TA* w, const float* bias, TC* c, int m, int n, int k, cudaStream_t stream) {
+    const dim3 large((n + 63) / 64, (m + 63) / 64);
+    if ((long long)large.x * large.y >= 148) return launch(gemm_tile_kernel<TA, TC, 64, 8>, large, 64, 0, stream, a, w, bias, c, m, n, k);
+    return launch(gemm_tile_kernel<TA, TC, 32, 4>, dim3((n + 31) / 32, (m + 31) / 32), 64, 0, stream, a, w, bias, c, m, n, k);
+}
+
+template <typename TA, typename TC>
+cudaError_t launch_typed(const TA* a, const TA* w, const float* bias, TC* c, int m, int n, int k, cudaStream_t stream) {
+    // (the ring's copies are of 16 bytes: operands that begin elsewhere, which only bfloat16 views can, take the tiles)
+    const bool aligned = (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
+    if (m > (n >= kStreamFourRows ? kStreamRowsWide : kStreamRows) || !aligned) return launch_tile<TA, TC>(a, w, bias, c, m, n, k, stream);
+    if (m == 1) return launch_stream<TA, TC, 1>(a, w, bias, c, m, n, k, stream);
+    if (m == 2) return launch_stream<TA, TC, 2>(a, w, bias, c, m, n, k, stream);
+    if (m <= 4) return launch_stream<TA, TC, 4>(a, w, bias, c, m, n, k, stream);
+    return launch_stream<TA, TC, 8>(a, w, bias, c, m, n, k, stream);
+}
+}  // namespace
+
 cudaError_t launch_gemm_simt(int in_dtype, int out_dtype, const void* a, const void* w, const float* bias, void* c,
                              int m, int n, int k, cudaStream_t stream) {
     if (m == 0 || n == 0) return cudaSuccess;
-    dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
     if (in_dtype == kF32 && out_dtype == kF32)
-        return launch(gemm_simt_kernel<float, float>, grid, 256, 0, stream, (const float*)a, (const float*)w, bias, (float*)c, m, n, k);
+        return launch_typed<float, float>((const float*)a, (const float*)w, bias, (float*)c, m, n, k, stream);
     if (in_dtype == kBF16 && out_dtype == kBF16)
-        return launch(gemm_simt_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, stream,
-            (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)c, m, n, k);
+        return launch_typed<__nv_bfloat16, __nv_bfloat16>((const __nv_bfloat16*)a, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)c, m, n, k, stream);
     if (in_dtype == kBF16 && out_dtype == kF32)
-        return launch(gemm_simt_kernel<__nv_bfloat16, float>, grid, 256, 0, stream,
-            (const __nv_bfloat16*)a, (const __nv_bfloat16*)w, bias, (float*)c, m, n, k);
+        return launch_typed<__nv_bfloat16, float>((const __nv_bfloat16*)a, (const __nv_bfloat16*)w, bias, (float*)c, m, n, k, stream);
     return cudaErrorInvalidValue;
 }
 
