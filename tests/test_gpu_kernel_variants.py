@@ -35,3 +35,39 @@ def test_32_bit_products_are_the_same_in_both_kernels(n, k):
     for m in (1, 2, 3, 4, 5, 8, 9, 31, 32, 33, 64, 65, 129):
         part = ops().linear(a[:m].contiguous(), w, bias, torch.full((m, n), float("nan"), device=DEV))
         assert torch.equal(part, whole[:m]), m
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,page,window", [(14, 2, 64, 64, None), (9, 1, 64, 16, 40), (3, 3, 128, 32, None), (8, 1, 128, 16, 33),
+                                                          (4, 2, 80, 16, 32), (2, 1, 256, 16, None), (6, 3, 192, 48, 31), (5, 1, 16, 16, 1)])
+def test_32_bit_attention_at_the_edges_of_its_segments(heads, kv_heads, d, page, window):
+    """Keys in one segment of 32, at its border, in all warps and beyond; a token alone equals the token in a portion bit for bit."""
+    g = torch.Generator().manual_seed(heads + d)
+    lens = [1, 31, 32, 33, 255, 256, 257, 300]
+    q_lens = [1, 5, 1, 2, 1, 3, 1, 40]
+    k, v = (torch.randn((sum(lens), kv_heads, d), generator=g) for _ in range(2))
+    kc, vc, table = paged_cache(k, v, lens, page, sum(-(-n // page) for n in lens) + 3, torch.float32, seed=2)
+    T = sum(q_lens)
+    q = torch.randn((T, heads, d), generator=g) * 2
+    qkv = torch.cat([q.view(T, -1), torch.zeros(T, 2 * kv_heads * d)], dim=1).to(DEV)
+    starts = [n - m for n, m in zip(lens, q_lens)]
+    status = torch.zeros(2, dtype=torch.int32, device=DEV)
+    out = torch.full((T, heads * d), float("nan"), device=DEV)
+    scale = 1 / math.sqrt(d)
+    ops().paged_attention(qkv, out, kc, vc, helpers.step_context(q_lens, starts, DEV), table, heads, kv_heads, d, window, scale, status=status)
+    assert status.tolist() == [0, 0]
+    at_q = at_k = 0
+    for s, (n, m) in enumerate(zip(lens, q_lens)):
+        qq = torch.zeros((n, heads, d), dtype=F)
+        qq[n - m:] = q[at_q:at_q + m].double()
+        ref = plain.attention(qq, k[at_k:at_k + n].double(), v[at_k:at_k + n].double(), window)[n - m:]
+        assert float((out[at_q:at_q + m].cpu().double().view(m, heads, d) - ref).abs().max()) <= 2e-5, s
+        alone = torch.empty((1, heads * d), device=DEV)
+        ops().paged_attention(qkv[at_q + m - 1:at_q + m], alone, kc, vc, helpers.step_context([1], [n - 1], DEV), table[s:s + 1], heads, kv_heads,
+                              d, window, scale)
+        assert torch.equal(alone[0], out[at_q + m - 1])
+        at_q, at_k = at_q + m, at_k + n
+    # a page that the table does not name sets the status word; the other keys count
+    bad = table.clone()
+    bad[7, 0] = -1
+    ops().paged_attention(qkv, out, kc, vc, helpers.step_context(q_lens, starts, DEV), bad, heads, kv_heads, d, None, scale, status=status)
+    assert status.tolist() == [3, -1] and bool(torch.isfinite(out).all())

@@ -1,4 +1,4 @@
-// Attention over the paged cache, one warp for a (token, head): the plain kernel.
+// Attention over the paged cache in 32-bit arithmetic without tensor cores: the plain kernel.
 //
 // It is the whole 32-bit path and the fallback of the bfloat16 path for head sizes the
 // tensor-core kernels do not take.  What it computes is vt-transformer's chain
@@ -7,8 +7,14 @@
 // P V (cuda_tensor.cpp:869-881), with the KV head of a query head being head / group
 // (v1/tensortype/cuda_kernels/transpose_0213.cu:93-105) -- but without the [heads, T, F]
 // score tensor, the repeated heads or the dense copy of the cache: the keys are read where
-// they lie in their pages, one after the other in the order of their positions, with a
-// running maximum and sum in 32-bit.  The result for a token depends on its own keys only.
+// they lie in their pages.
+//
+// A CTA serves a token and the heads of one KV group (up to kHeads of them), so that a key or value is fetched once for
+// all of them.  The keys are cut into segments of 32 by their absolute positions; warp w takes every eighth segment (every fourth
+// for heads of more than 128 numbers) from the w-th on, in order: the 32 keys go through shared memory, a lane forms its key's scores, and the lanes then take the dimensions
+// of the values.  Each warp keeps a running maximum, sum and result a head, in 32-bit; the warps' are put together at
+// the end in the order of the warps.  Which warp adds what in which order depends on the token's position and the
+// window alone, so a token's result depends on its own keys only, however the tokens are cut into steps.
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.cuh"
@@ -16,78 +22,236 @@
 namespace vtb {
 
 namespace {
-constexpr int kMaxPerLane = 8;   // head_dim <= 256
+constexpr int kSegment = 32;         // keys a warp takes at once
+// Warps of a CTA, by the dimensions a lane holds (heads of more than 128 numbers leave shared memory for four segments).
+__host__ __device__ constexpr int warps_of(int per_lane) { return per_lane > 4 ? 4 : 8; }
+constexpr int kHeadDimMax = 256;
+
+// Four consecutive numbers as floats; the address is a multiple of 4 elements.
+__device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(128)
+// Shared memory of a CTA, in floats: q of the heads, each warp's segment of keys (rows `row` floats apart, later the
+// warp's results), each warp's weights.
+__host__ __device__ inline int padded_dim(int head_dim) { return (head_dim + 3) / 4 * 4; }
+__host__ __device__ inline int key_row(int head_dim) { return padded_dim(head_dim) + 4; }
+__host__ __device__ inline int smem_floats(int head_dim, int heads, int warps) {
+    return heads * padded_dim(head_dim) + warps * (kSegment * key_row(head_dim) + heads * kSegment);
+}
+}  // namespace
+
+template <typename T, int HEADS, int PER_LANE>
+__global__ void __launch_bounds__(32 * warps_of(PER_LANE))
 attention_simt_kernel(const T* __restrict__ qkv, int qkv_stride, T* __restrict__ out, const T* __restrict__ k_cache,
                       const T* __restrict__ v_cache, const int* __restrict__ positions,
                       const int* __restrict__ token_seq, const int* __restrict__ block_table, int table_stride,
-                      int n_seqs, int n_pages, int n_tokens, int heads, int kv_heads, int head_dim, int page_size,
+                      int n_seqs, int n_pages, int heads, int kv_heads, int head_dim, int page_size,
                       int window, float scale, int* status) {
+    constexpr int kWarps = warps_of(PER_LANE);
+    extern __shared__ __align__(16) float smem[];
     pdl_launch();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const long long pair = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (pair >= (long long)n_tokens * heads) return;
-    const int t = (int)(pair / heads), h = (int)(pair % heads);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int group = heads / kv_heads, per_kv = (group + HEADS - 1) / HEADS;
+    const int t = blockIdx.x, kvh = blockIdx.y / per_kv;
+    const int h0 = kvh * group + (blockIdx.y % per_kv) * HEADS;       // the CTA's first head, and how many it has
+    const int nh = min(HEADS, (kvh + 1) * group - h0);
+    const int dim4 = padded_dim(head_dim), row = key_row(head_dim);
     const int seq = token_seq[t];
-    T* o = out + (size_t)t * heads * head_dim + (size_t)h * head_dim;
+    T* o = out + (size_t)t * heads * head_dim + (size_t)h0 * head_dim;
     if (seq < 0) {   // padding
-        for (int i = lane; i < head_dim; i += 32) o[i] = from_float<T>(0.f);
+        for (int i = threadIdx.x; i < nh * head_dim; i += blockDim.x) o[i] = from_float<T>(0.f);
         return;
     }
     if (seq >= n_seqs) {
-        if (lane == 0) set_status(status, kStatusBadSequence, seq);
+        if (threadIdx.x == 0) set_status(status, kStatusBadSequence, seq);
         return;
     }
     const int pos = positions[t];
-    const int kvh = h / (heads / kv_heads);
     const int* table = block_table + (size_t)seq * table_stride;
+    float* qs = smem;
+    float* keys = smem + HEADS * dim4 + warp * (kSegment * row);
+    float* ps = smem + HEADS * dim4 + kWarps * (kSegment * row) + warp * (HEADS * kSegment);
+    const T* qp = qkv + (size_t)t * qkv_stride + (size_t)h0 * head_dim;
+    for (int i = threadIdx.x; i < HEADS * dim4; i += blockDim.x) {
+        const int g = i / dim4, d = i - g * dim4;
+        qs[i] = (g < nh && d < head_dim) ? to_float(qp[g * head_dim + d]) : 0.f;
+    }
+    __syncthreads();
 
-    float q[kMaxPerLane], acc[kMaxPerLane];
-    const T* qp = qkv + (size_t)t * qkv_stride + (size_t)h * head_dim;
+    float acc[HEADS][PER_LANE], mx[HEADS], sum[HEADS];
 #pragma unroll
-    for (int r = 0; r < kMaxPerLane; ++r) {
-        const int i = lane + 32 * r;
-        q[r] = (i < head_dim) ? to_float(qp[i]) : 0.f;
-        acc[r] = 0.f;
+    for (int g = 0; g < HEADS; ++g) {
+        mx[g] = -INFINITY;
+        sum[g] = 0.f;
+#pragma unroll
+        for (int r = 0; r < PER_LANE; ++r) acc[g][r] = 0.f;
     }
-    float mx = -INFINITY, sum = 0.f;
     const int first = (window > 0) ? max(0, pos - window + 1) : 0;
-    for (int j = first; j <= pos; ++j) {
-        const int page = table[j / page_size];
-        if (page < 0 || page >= n_pages) {
-            if (lane == 0) set_status(status, kStatusBadPage, page);
-            continue;
+    const int seg_first = first / kSegment, seg_last = pos < 0 ? -1 : pos / kSegment;
+    for (int seg = seg_first / kWarps * kWarps + warp; seg <= seg_last; seg += kWarps) {
+        if (seg < seg_first) continue;
+        const int j = seg * kSegment + lane;
+        bool seen = j >= first && j <= pos;
+        long long base = 0;
+        if (seen) {
+            const int page = table[j / page_size];
+            if (page < 0 || page >= n_pages) {
+                set_status(status, kStatusBadPage, page);
+                seen = false;
+            } else {
+                base = (((long long)page * kv_heads + kvh) * page_size + (j % page_size)) * head_dim;
+            }
         }
-        const size_t base = (((size_t)page * kv_heads + kvh) * page_size + (j % page_size)) * head_dim;
-        float part = 0.f;
+        const unsigned mask = __ballot_sync(0xffffffffu, seen);
+        if (mask == 0) continue;
+        // the keys' rows into shared memory (those that are not seen as zeros: their memory may hold anything)
+        if ((head_dim & 3) == 0) {
+            const int quads = head_dim >> 2;
+            int r = 0, q = lane;
+#pragma unroll 8
+            for (int e = 0; e < quads; ++e) {          // 32 rows of `quads` pieces, 32 pieces at a time
+                while (q >= quads) { q -= quads; ++r; }
+                const long long b = __shfl_sync(0xffffffffu, base, r);
+                const float4 v = (mask >> r & 1) ? four(k_cache + b + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(keys + r * row + 4 * q) = v;
+                q += 32;
+            }
+        } else {
+            for (int r = 0; r < kSegment; ++r) {
+                const long long b = __shfl_sync(0xffffffffu, base, r);
+                for (int d = lane; d < dim4; d += 32)
+                    keys[r * row + d] = (d < head_dim && (mask >> r & 1)) ? to_float(k_cache[b + d]) : 0.f;
+            }
+        }
+        __syncwarp();
+        // a lane's key against every head: four chains over the dimensions
+        float4 dot[HEADS];
 #pragma unroll
-        for (int r = 0; r < kMaxPerLane; ++r) {
-            const int i = lane + 32 * r;
-            if (i < head_dim) part = fmaf(q[r], to_float(k_cache[base + i]), part);
-        }
-        const float s = warp_sum(part) * scale;
-        const float new_mx = fmaxf(mx, s);
-        const float corr = expf(mx - new_mx);   // 0 at the first key (mx = -inf)
-        const float p = expf(s - new_mx);
-        sum = sum * corr + p;
+        for (int g = 0; g < HEADS; ++g) dot[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int d = 0; d < dim4; d += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(keys + lane * row + d);
 #pragma unroll
-        for (int r = 0; r < kMaxPerLane; ++r) {
-            const int i = lane + 32 * r;
-            if (i < head_dim) acc[r] = acc[r] * corr + p * to_float(v_cache[base + i]);
+            for (int g = 0; g < HEADS; ++g) {
+                const float4 qv = *reinterpret_cast<const float4*>(qs + g * dim4 + d);
+                dot[g].x = fmaf(qv.x, kv.x, dot[g].x);
+                dot[g].y = fmaf(qv.y, kv.y, dot[g].y);
+                dot[g].z = fmaf(qv.z, kv.z, dot[g].z);
+                dot[g].w = fmaf(qv.w, kv.w, dot[g].w);
+            }
         }
-        mx = new_mx;
+#pragma unroll
+        for (int g = 0; g < HEADS; ++g) {              // (of a group of fewer heads the last ones are zeros that nothing reads)
+            const float s = seen ? ((dot[g].x + dot[g].y) + (dot[g].z + dot[g].w)) * scale : -INFINITY;
+            const float new_mx = fmaxf(mx[g], warp_max(s));
+            const float p = seen ? expf(s - new_mx) : 0.f;
+            const float corr = mx[g] == -INFINITY ? 0.f : expf(mx[g] - new_mx);      // (0 at the warp's first keys)
+            sum[g] = sum[g] * corr + warp_sum(p);
+            mx[g] = new_mx;
+#pragma unroll
+            for (int r = 0; r < PER_LANE; ++r) acc[g][r] *= corr;
+            ps[g * kSegment + lane] = p;
+        }
+        __syncwarp();
+        // the values, a row after the other in the order of the positions, eight rows on their way at once (a key that is not
+        // seen weighs 0 and counts with a value of 0)
+        for (int r0 = 0; r0 < kSegment; r0 += 8) {
+            if ((mask >> r0 & 0xffu) == 0) continue;
+            float v[8][PER_LANE];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const long long b = __shfl_sync(0xffffffffu, base, r0 + r);
+                const bool in = mask >> (r0 + r) & 1;
+#pragma unroll
+                for (int i = 0; i < PER_LANE; ++i) v[r][i] = (in && lane + 32 * i < head_dim) ? to_float(v_cache[b + lane + 32 * i]) : 0.f;
+            }
+#pragma unroll
+            for (int g = 0; g < HEADS; ++g) {
+                const float4 p0 = *reinterpret_cast<const float4*>(ps + g * kSegment + r0);
+                const float4 p1 = *reinterpret_cast<const float4*>(ps + g * kSegment + r0 + 4);
+                const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+#pragma unroll
+                    for (int i = 0; i < PER_LANE; ++i) acc[g][i] = fmaf(p[r], v[r][i], acc[g][i]);
+            }
+        }
+        __syncwarp();
     }
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    // the warps' results: [head][dimension], then the maximum and the sum
+    __syncwarp();
 #pragma unroll
-    for (int r = 0; r < kMaxPerLane; ++r) {
-        const int i = lane + 32 * r;
-        if (i < head_dim) o[i] = from_float<T>(acc[r] * inv);
+    for (int g = 0; g < HEADS; ++g) {
+        if (g >= nh) break;
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i)
+            if (lane + 32 * i < head_dim) keys[g * (dim4 + 2) + lane + 32 * i] = acc[g][i];
+        if (lane == 0) {
+            keys[g * (dim4 + 2) + dim4] = mx[g];
+            keys[g * (dim4 + 2) + dim4 + 1] = sum[g];
+        }
+    }
+    __syncthreads();
+    const float* parts = smem + HEADS * dim4;
+    for (int i = threadIdx.x; i < nh * head_dim; i += blockDim.x) {
+        const int g = i / head_dim, d = i - g * head_dim;
+        const float* at = parts + g * (dim4 + 2);
+        float top = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) top = fmaxf(top, at[w * (kSegment * row) + dim4]);
+        float total = 0.f, value = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const float* pw = at + w * (kSegment * row);
+            if (pw[dim4 + 1] == 0.f) continue;                        // (a warp without keys)
+            const float f = expf(pw[dim4] - top);
+            total = fmaf(pw[dim4 + 1], f, total);
+            value = fmaf(pw[d], f, value);
+        }
+        const float inv = total > 0.f ? 1.f / total : (total == 0.f ? 0.f : total);      // (a NaN stays one)
+        o[i] = from_float<T>(value * inv);
     }
 }
+
+namespace {
+template <typename T, int HEADS, int PER_LANE>
+cudaError_t launch_one(dim3 grid, const T* qkv, int qkv_stride, T* out, const T* k_cache, const T* v_cache, const int* positions,
+                       const int* token_seq, const int* block_table, int table_stride, int n_seqs, int n_pages, int heads, int kv_heads,
+                       int head_dim, int page_size, int window, float scale, int* status, cudaStream_t stream) {
+    static std::atomic<unsigned long long> done{0};
+    const int most = smem_floats(32 * PER_LANE, HEADS, warps_of(PER_LANE)) * (int)sizeof(float);
+    const cudaError_t e = allow_dynamic_smem(attention_simt_kernel<T, HEADS, PER_LANE>, most, done);
+    if (e != cudaSuccess) return e;
+    return launch(attention_simt_kernel<T, HEADS, PER_LANE>, grid, 32 * warps_of(PER_LANE), smem_floats(head_dim, HEADS, warps_of(PER_LANE)) * sizeof(float), stream, qkv,
+                  qkv_stride, out, k_cache, v_cache, positions, token_seq, block_table, table_stride, n_seqs, n_pages, heads, kv_heads,
+                  head_dim, page_size, window, scale, status);
+}
+
+// Heads a CTA: all of a group of up to 7 (the sizes in use), fewer where the results would not fit a thread's registers
+// or the keys shared memory.
+template <typename T, typename... Args>
+cudaError_t launch_typed(int n_tokens, int heads, int kv_heads, int head_dim, Args... args) {
+    const int group = heads / kv_heads;
+    auto grid = [&](int per) { return dim3(n_tokens, kv_heads * ((group + per - 1) / per)); };
+    if (head_dim <= 64) {
+        if (group == 1) return launch_one<T, 1, 2>(grid(1), args...);
+        if (group <= 4) return launch_one<T, 4, 2>(grid(4), args...);
+        return launch_one<T, 7, 2>(grid(7), args...);
+    }
+    if (head_dim <= 128) {
+        if (group == 1) return launch_one<T, 1, 4>(grid(1), args...);
+        if (group <= 4) return launch_one<T, 4, 4>(grid(4), args...);
+        return launch_one<T, 7, 4>(grid(7), args...);
+    }
+    return launch_one<T, 1, 8>(grid(1), args...);
+}
+}  // namespace
 
 cudaError_t launch_attention_simt(int dtype, const void* qkv, int qkv_stride, void* out, const void* k_cache,
                                   const void* v_cache, const int* positions, const int* token_seq,
@@ -95,18 +259,16 @@ cudaError_t launch_attention_simt(int dtype, const void* qkv, int qkv_stride, vo
                                   int heads, int kv_heads, int head_dim, int page_size, int window, float scale,
                                   int* status, cudaStream_t stream) {
     if (n_tokens == 0) return cudaSuccess;
-    if (head_dim > 32 * kMaxPerLane) return cudaErrorInvalidValue;
-    const long long pairs = (long long)n_tokens * heads;
-    const int blocks = (int)((pairs + 3) / 4);
-    if (dtype == kBF16)
-        return launch(attention_simt_kernel<__nv_bfloat16>, blocks, 128, 0, stream,
-            (const __nv_bfloat16*)qkv, qkv_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_cache,
-            (const __nv_bfloat16*)v_cache, positions, token_seq, block_table, table_stride, n_seqs, n_pages, n_tokens,
-            heads, kv_heads, head_dim, page_size, window, scale, status);
-    return launch(attention_simt_kernel<float>, blocks, 128, 0, stream,
-            (const float*)qkv, qkv_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, positions,
-            token_seq, block_table, table_stride, n_seqs, n_pages, n_tokens, heads, kv_heads, head_dim, page_size,
-            window, scale, status);
+    if (head_dim > kHeadDimMax) return cudaErrorInvalidValue;
+    if (dtype == kBF16) {
+        using B = __nv_bfloat16;
+        return launch_typed<B>(n_tokens, heads, kv_heads, head_dim, (const B*)qkv, qkv_stride, (B*)out, (const B*)k_cache, (const B*)v_cache,
+                               positions, token_seq, block_table, table_stride, n_seqs, n_pages, heads, kv_heads, head_dim, page_size, window,
+                               scale, status, stream);
+    }
+    return launch_typed<float>(n_tokens, heads, kv_heads, head_dim, (const float*)qkv, qkv_stride, (float*)out, (const float*)k_cache,
+                               (const float*)v_cache, positions, token_seq, block_table, table_stride, n_seqs, n_pages, heads, kv_heads,
+                               head_dim, page_size, window, scale, status, stream);
 }
 
 }  // namespace vtb
