@@ -71,3 +71,48 @@ def test_32_bit_attention_at_the_edges_of_its_segments(heads, kv_heads, d, page,
     bad[7, 0] = -1
     ops().paged_attention(qkv, out, kc, vc, helpers.step_context(q_lens, starts, DEV), bad, heads, kv_heads, d, None, scale, status=status)
     assert status.tolist() == [3, -1] and bool(torch.isfinite(out).all())
+
+
+def walked(o, name, y, state, ctx, v_dim, heads, walk, call):
+    """One scan of ``ctx`` from ``state`` with the walking kernel or without it."""
+    out = torch.full((y.shape[0], heads * v_dim), float("nan"), device=DEV)
+    st = state.clone()
+    old = o.SCAN_WALK_THREADS
+    o.SCAN_WALK_THREADS = 256 if walk else 0
+    try:
+        call(st, out)
+    finally:
+        o.SCAN_WALK_THREADS = old
+    return out, st
+
+
+# (keys at both ends of each form, values in a part of a warp's 32 columns, in several warps and CTAs; tokens around a batch of 16)
+@pytest.mark.parametrize("dim,v_dim,heads", [(34, 32, 3), (64, 64, 2), (64, 136, 5), (66, 40, 2), (128, 256, 2), (120, 90, 40)])
+@pytest.mark.parametrize("lens", [[1, 16, 47], [17, 33, 15, 100]])
+def test_walks_along_portions_equal_the_token_by_token_kernel(dim, v_dim, heads, lens):
+    """Gated linear attention, delta rule and retention in bfloat16 portions: results and last states of both kernels, whose sums differ
+    in their order alone (32-bit sums of up to 128 terms, and what a recurrence of 100 tokens makes of them)."""
+    o, rank = ops(), 16
+    g = torch.Generator().manual_seed(dim + v_dim)
+    T, n = sum(lens), len(lens)
+    ctx = helpers.step_context(lens, [3] * n, DEV)
+    rnd = lambda *s: torch.randn(s, generator=g).to(DEV)
+    rows = n + 1
+    q_col, k_col, a_col, low_col = 0, heads * dim, 2 * heads * dim, 3 * heads * dim
+    v_col = low_col + rank
+    y = (rnd(T, v_col + heads * max(v_dim, dim) + (heads * max(v_dim, dim)) % 2) * 0.5).to(torch.bfloat16)
+    w2, b2, ab = rnd(heads * dim, rank) * 0.3, rnd(heads * dim), rnd(heads * dim)
+    decay = torch.linspace(0.5, 0.999, heads).to(DEV)
+    freq = torch.linspace(1.0, 0.01, dim // 4).to(DEV)
+    cases = {
+        "gla": (v_dim, lambda st, out: o.gla_scan(y, q_col, k_col, v_col, low_col, w2, b2, 1 / 16, dim ** -0.5, st, ctx, out, heads, dim, v_dim)),
+        "delta": (dim, lambda st, out: o.delta_scan(y, q_col, k_col, v_col, a_col, low_col, w2, b2, ab, math.exp(-0.5), 1e-6, st, ctx, out, heads, dim)),
+        "retention": (v_dim, lambda st, out: o.retention_scan(y, q_col, k_col, v_col, decay, dim ** -0.5, freq, st, ctx, out, heads, dim, v_dim, act=True)),
+    }
+    for name, (cols, call) in cases.items():
+        state = rnd(rows, heads, dim, cols)
+        got, last = walked(o, name, y, state, ctx, cols, heads, True, call)
+        ref, ref_last = walked(o, name, y, state, ctx, cols, heads, False, call)
+        for a, b in ((got, ref), (last, ref_last)):
+            assert float((a - b).abs().max()) <= 2e-5 * max(1.0, float(b.abs().max())), name
+        assert torch.equal(last[n:], state[n:])            # a row of no sequence of the step

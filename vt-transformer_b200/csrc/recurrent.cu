@@ -370,8 +370,22 @@ cudaError_t launch_scan_kd(ScanArgs a, int n_seqs, cudaStream_t stream) {
     return launch(scan_kernel<T, KD, Delta, Walk, Fixed>, grid, block, bytes, stream, a);
 }
 
+}  // namespace
+
+}  // namespace vtb
+
+#include "recurrent_walk.cuh"
+
+namespace vtb {
+
+namespace {
+
 template <typename T, bool Delta, bool Fixed = false>
 cudaError_t launch_scan_t(ScanArgs a, int n_seqs, cudaStream_t stream) {
+    if constexpr (sizeof(T) == 2) {
+        if (walk_takes(a) && walk_smem_floats<8, Delta, Fixed>(a.dim, a.rank, 128) * 4 <= 200 * 1024)
+            return a.dim <= 64 ? launch_scan_walk<T, 4, Delta, Fixed>(a, n_seqs, stream) : launch_scan_walk<T, 8, Delta, Fixed>(a, n_seqs, stream);
+    }
     // Rows a thread: 16 where that makes at most 8 groups of warps a column, else 32, 64, 128.  Few rows a thread make
     // the walk along the tokens short (a token costs a thread rows / 4 steps of loads and multiply-adds, whatever the
     // number of groups), which is what bounds a sequence's portion of a prompt; the groups' shares meet in shared memory.

@@ -1,0 +1,336 @@
+// The recurrences of recurrent.cu along a portion of a prompt in bfloat16 steps, for keys of 33 to 128 numbers.
+//
+// What bounds the walk is a sequence's own chain: a token's multiply-adds, the numbers that shared memory delivers for
+// them (a warp's 16-byte load takes four cycles whatever its lanes share) and the meeting of the threads that hold a
+// column.  A thread here holds 16 rows of CPT columns, so that a number of q, k or the decay that it loads serves CPT
+// multiply-adds, and the RG threads that share a column are neighbours in one warp: they meet by shuffles, no barrier
+// stands inside a token.  Four more warps stage the next 16 tokens (loads, gates, unit keys, rotation) while the others
+// walk.  State, gates and sums are 32-bit as in scan_kernel; only the order of the sums over a column differs, which is why
+// a 32-bit step, whose tokens must not depend on what else is in the step, stays with scan_kernel.
+//
+// Measured on a B200, us, scan_kernel's walk and this one: 4 sequences of up to 1,500 tokens, 8 heads: gated linear attention of
+// 64 x 128 1,119 and 722, delta rule of 64 x 64 1,755 and 960; retention of 16 heads of 128 x 256 over 4,096 tokens in segments 1,471 and
+// 580.  Four columns a thread for keys of more than 64 numbers (twice the warps, half the registers) were slower: 634.
+#pragma once
+
+namespace vtb {
+
+namespace {
+
+constexpr int kWalkTokens = 16;       // tokens staged at once
+constexpr int kWalkStagers = 128;     // threads that stage
+constexpr int kWalkWarps = 4;         // the most warps that walk (with eight rows of pairs by eight columns a thread, all registers)
+
+struct Pair { unsigned long long v; };           // two floats that are computed with together
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void pair_halves(Pair a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(a.v)); }
+__device__ __forceinline__ float pair_sum(Pair a) {
+    float lo, hi;
+    pair_halves(a, lo, hi);
+    return lo + hi;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// Numbers of a staged token: q, k, then the decay (not with Fixed), then b = a u and u (Delta); the values lie apart.
+template <bool Delta, bool Fixed> __host__ __device__ constexpr int walk_vectors() { return Delta ? 5 : (Fixed ? 2 : 3); }
+
+template <int RG, bool Delta, bool Fixed>
+__host__ __device__ inline int walk_smem_floats(int dim, int rank, int cols) {
+    return ((dim * rank + 3) & ~3) + ((kWalkTokens * rank + 3) & ~3) + 2 * kWalkTokens * (walk_vectors<Delta, Fixed>() * 16 * RG + cols);
+}
+
+// RG: the threads that share a column (16 rows each); they hold CPT = RG columns each, so a warp has 32.
+template <typename T, int RG, bool Delta, bool Fixed>
+__global__ void __launch_bounds__(kWalkStagers + 32 * kWalkWarps, 1)
+scan_walk_kernel(const ScanArgs a) {
+    constexpr int CPT = RG, DP = 16 * RG, TB = kWalkTokens, VEC = walk_vectors<Delta, Fixed>();
+    constexpr int D_AT = 2, B_AT = 3, U_AT = 4;
+    extern __shared__ __align__(16) float smem[];
+    pdl_launch();
+    const int seq = blockIdx.x, h = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int walkers = blockDim.x - kWalkStagers, cols = walkers;          // a column a walking thread
+    const int dim = a.dim, v_dim = a.v_dim, rank = a.rank, col0 = blockIdx.z * cols;
+    float* w2s = smem;                                                      // [dim, rank]: the low-rank gate's second matrix
+    float* low = w2s + ((dim * rank + 3) & ~3);                             // [tokens, rank]
+    float* stage = low + ((TB * rank + 3) & ~3);                            // [2][tokens][VEC][DP], then [2][tokens][cols]
+    float* values = stage + 2 * TB * VEC * DP;
+    // the weights are written by no kernel of the step: they are read before the wait
+    for (int e = tid; e < dim * rank; e += blockDim.x) w2s[e] = a.w2[(size_t)h * dim * rank + e];
+    pdl_wait();
+    const int t0 = a.cu_q[seq], t1 = a.cu_q[seq + 1];
+    if (t1 <= t0) return;                                   // a sequence without tokens in this step (padding): its state stays
+    const int row = a.rows[seq];
+    const bool later = Fixed && row < 0 && a.ends != nullptr;      // a later segment of a walk that was cut
+    if (later ? (-row - 1 >= a.end_rows) : (row < 0 || row >= a.state_rows)) {
+        if (tid == 0) set_status(a.status, kStatusBadRow, row);
+        return;
+    }
+    float* sp = later ? a.ends + (((size_t)(-row - 1) * a.heads + h) * dim) * v_dim
+                      : a.state + (((size_t)row * a.heads + h) * dim) * v_dim;
+    const T* y = reinterpret_cast<const T*>(a.y);
+    const int batches = (t1 - t0 + TB - 1) / TB;
+    const int st = tid - walkers;                           // a staging thread's number (negative: it walks)
+    __syncthreads();
+
+    // a walking thread: rows 4 (rg + RG i) .. + 3 for i = 0..3 of the columns wc .. wc + CPT - 1 of this CTA
+    const int rg = lane % RG, wc = (tid & ~31) + lane / RG * CPT;
+    Pair S[8][CPT];                                         // [pair of rows][column]
+    if (st < 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                const int r = 4 * (rg + RG * (i >> 1)) + 2 * (i & 1), j = col0 + wc + c;
+                const bool in = !later && j < v_dim;
+                S[i][c] = pair_of(in && r < dim ? sp[(size_t)r * v_dim + j] : 0.f, in && r + 1 < dim ? sp[(size_t)(r + 1) * v_dim + j] : 0.f);
+            }
+    }
+    const float decay = Fixed ? a.bias2[h] : 0.f;
+
+    // ---- staging ----------------------------------------------------------------------------------------------
+    // two neighbouring numbers of a token at a time: q, k and (Delta) the removal rate, each DP wide, the gate's input, the values
+    constexpr int kRead = Delta ? 3 : 2;
+    const int pairs = (kRead * DP + cols + rank) / 2;
+    auto stage_batch = [&](int batch) {
+        const int first = t0 + batch * TB, n = min(TB, t1 - first);
+        float* to = stage + (batch & 1) * TB * VEC * DP;
+        float* vto = values + (batch & 1) * TB * cols;
+        for (int s = st; s < pairs; s += kWalkStagers) {
+            const int r = 2 * s;
+            int from = -1, step;
+            float* dst;
+            float times = 1.f;
+            bool act = Fixed && a.act != 0;
+            if (r < kRead * DP) {
+                const int which = r / DP, i = r - which * DP;
+                if (i < dim) from = (which == 0 ? a.q_col : (which == 1 ? a.k_col : a.a_col)) + h * dim + i;
+                if (!Delta && which == (Fixed ? 1 : 0)) times = a.c2;
+                dst = to + (which == 2 ? B_AT : which) * DP + i;
+                step = VEC * DP;
+            } else if (r < kRead * DP + cols) {
+                const int i = r - kRead * DP;
+                if (col0 + i < v_dim) from = a.v_col + h * v_dim + col0 + i;
+                dst = vto + i;
+                step = cols;
+            } else {
+                const int i = r - kRead * DP - cols;
+                from = a.low_col + i;
+                dst = low + i;
+                step = rank;
+                act = false;
+            }
+            const bool is_low = r >= kRead * DP + cols;
+            const T* src = y + (size_t)first * a.stride + (from < 0 ? 0 : from);
+            float2 val[TB];
+#pragma unroll
+            for (int t = 0; t < TB; ++t) {
+                const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(src + (size_t)min(t, n - 1) * a.stride);
+                val[t] = from < 0 ? make_float2(0.f, 0.f) : __bfloat1622float2(b);
+            }
+#pragma unroll
+            for (int t = 0; t < TB; ++t) {
+                if (t >= n) break;
+                float2 v = val[t];
+                if (act) {
+                    v.x = v.x / (1.f + expf(-v.x));
+                    v.y = v.y / (1.f + expf(-v.y));
+                }
+                v.x *= times;
+                v.y *= times;
+                if (Delta && is_low) {
+                    v.x = tanhf(v.x);
+                    v.y = tanhf(v.y);
+                }
+                *reinterpret_cast<float2*>(dst + t * step) = v;
+            }
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kWalkStagers) : "memory");
+        if (Fixed) {
+            // the rotation of q and k: a thread turns both members of a pair, so nothing else touches them meanwhile
+            const int half = a.half;
+            for (int e = st; e < n * half; e += kWalkStagers) {
+                const int t = e / half, i = e % half;
+                float sn, cs;
+                sincosf((float)a.positions[first + t] * a.freq[i], &sn, &cs);
+                float* qv = to + t * VEC * DP;
+                float* kv = qv + DP;
+                const float qa = qv[i], qb = qv[i + half], ka = kv[i], kb = kv[i + half];
+                qv[i] = qa * cs - qb * sn;
+                qv[i + half] = qb * cs + qa * sn;
+                kv[i] = ka * cs - kb * sn;
+                kv[i + half] = kb * cs + ka * sn;
+            }
+        } else {
+            for (int e = st; e < n * DP; e += kWalkStagers) {
+                const int t = e / DP, i = e % DP;
+                float d = 0.f;
+                if (i < dim) {
+                    const int ch = h * dim + i;
+                    float z = a.bias2[ch];
+                    const float* wr = w2s + i * rank;
+                    const float* lr = low + t * rank;
+                    for (int r = 0; r < rank; ++r) z = fmaf(wr[r], lr[r], z);
+                    if (Delta) {
+                        d = expf(-a.c1 * sigmoid(z));
+                        float* b = to + t * VEC * DP + B_AT * DP + i;
+                        *b = sigmoid(*b + a.a_bias[ch]);
+                    } else {
+                        d = expf(a.c1 * log_sigmoid(z));
+                    }
+                }
+                to[t * VEC * DP + D_AT * DP + i] = d;
+            }
+        }
+        if (Delta) {
+            asm volatile("bar.sync 1, %0;" ::"n"(kWalkStagers) : "memory");
+            // the unit key u = k / sqrt(sum(k^2) + eps), and b = a * u: a warp for each staged token
+            for (int t = st >> 5; t < n; t += kWalkStagers / 32) {
+                float* at = to + t * VEC * DP;
+                float ss = 0.f;
+                for (int i = lane; i < DP; i += 32) ss = fmaf(at[DP + i], at[DP + i], ss);
+                const float inv = 1.f / sqrtf(warp_sum(ss) + a.c2);
+                for (int i = lane; i < DP; i += 32) {
+                    const float u = at[DP + i] * inv;
+                    at[U_AT * DP + i] = u;
+                    at[B_AT * DP + i] *= u;
+                }
+            }
+        }
+    };
+
+    // ---- the walk -----------------------------------------------------------------------------------------------
+    auto walk_batch = [&](int batch) {
+        const int first = t0 + batch * TB, n = min(TB, t1 - first);
+        const float* at = stage + (batch & 1) * TB * VEC * DP + 4 * rg;
+        const float* vat = values + (batch & 1) * TB * cols + wc;
+        const int j = col0 + wc + rg;                       // the column whose sum this lane ends up with
+        float* o = a.out + (size_t)first * a.heads * v_dim + h * v_dim + j;
+        const Pair fixed = pair_of(decay, decay);
+        for (int t = 0; t < n; ++t, at += VEC * DP, vat += cols, o += a.heads * v_dim) {
+            Pair v[CPT], acc[CPT], gone[CPT];
+#pragma unroll
+            for (int c = 0; c < CPT; c += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(vat + c);
+                v[c] = pair_of(x.x, x.x); v[c + 1] = pair_of(x.y, x.y); v[c + 2] = pair_of(x.z, x.z); v[c + 3] = pair_of(x.w, x.w);
+            }
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) acc[c].v = gone[c].v = 0ull;
+            if (Delta) {
+                // u^T S of the old state: this thread's rows, then the RG threads of the column
+                Pair part[CPT];
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) part[c].v = 0ull;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(at + U_AT * DP + 4 * RG * i);
+#pragma unroll
+                    for (int c = 0; c < CPT; ++c) {
+                        part[c] = pair_fma({u.x}, S[2 * i][c], part[c]);
+                        part[c] = pair_fma({u.y}, S[2 * i + 1][c], part[c]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) {
+                    float s = pair_sum(part[c]);
+#pragma unroll
+                    for (int x = RG / 2; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+                    gone[c] = pair_of(-s, -s);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(at + 4 * RG * i);
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(at + DP + 4 * RG * i);
+                ulonglong2 d = make_ulonglong2(fixed.v, fixed.v), b = make_ulonglong2(0ull, 0ull);
+                if (!Fixed) d = *reinterpret_cast<const ulonglong2*>(at + D_AT * DP + 4 * RG * i);
+                if (Delta) b = *reinterpret_cast<const ulonglong2*>(at + B_AT * DP + 4 * RG * i);
+                const Pair qs[2] = {{q.x}, {q.y}}, ks[2] = {{k.x}, {k.y}}, ds[2] = {{d.x}, {d.y}}, bs[2] = {{b.x}, {b.y}};
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int c = 0; c < CPT; ++c) {
+                        const Pair add = Delta ? pair_fma(ks[p], v[c], pair_mul(bs[p], gone[c])) : pair_mul(ks[p], v[c]);
+                        S[2 * i + p][c] = pair_fma(ds[p], S[2 * i + p][c], add);
+                        acc[c] = pair_fma(S[2 * i + p][c], qs[p], acc[c]);
+                    }
+            }
+            // the RG threads of a column add up: each round halves the columns that a thread still has
+            float s[CPT];
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) s[c] = pair_sum(acc[c]);
+#pragma unroll
+            for (int x = RG / 2; x > 0; x >>= 1) {
+                const bool upper = rg & x;
+#pragma unroll
+                for (int c = 0; c < x; ++c) {
+                    const float give = upper ? s[c] : s[c + x], keep = upper ? s[c + x] : s[c];
+                    s[c] = keep + __shfl_xor_sync(0xffffffffu, give, x);
+                }
+            }
+            if (j < v_dim) *o = s[0];
+        }
+    };
+
+    for (int it = 0; it <= batches; ++it) {
+        if (st >= 0) {
+            if (it < batches) stage_batch(it);
+        } else if (it > 0) {
+            walk_batch(it - 1);
+        }
+        __syncthreads();
+    }
+    if (st < 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) {
+                const int r = 4 * (rg + RG * (i >> 1)) + 2 * (i & 1), j = col0 + wc + c;
+                float lo, hi;
+                pair_halves(S[i][c], lo, hi);
+                if (j < v_dim && r < dim) sp[(size_t)r * v_dim + j] = lo;
+                if (j < v_dim && r + 1 < dim) sp[(size_t)(r + 1) * v_dim + j] = hi;
+            }
+    }
+}
+
+// Whether the walk of a step goes through scan_walk_kernel: pairs of neighbouring numbers must be 4-byte aligned and lie
+// in one part of a row.
+inline bool walk_takes(const ScanArgs& a) {
+    return a.most_threads > 0 && a.dim > 32 && a.dim <= 128 && a.dim % 2 == 0 && a.v_dim % 2 == 0 && a.rank % 2 == 0 && a.stride % 2 == 0 &&
+           ((a.q_col | a.k_col | a.v_col | a.a_col | a.low_col) & 1) == 0 && ((uintptr_t)a.y & 3) == 0;
+}
+
+template <typename T, int RG, bool Delta, bool Fixed>
+cudaError_t launch_scan_walk(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
+    static std::atomic<unsigned long long> done{0};
+    // warps of 32 columns a CTA: as few as keep the CTAs within one round (each stages its tokens for itself)
+    const int col_warps = (a.v_dim + 31) / 32;
+    int warps = 1;
+    while (warps < kWalkWarps && (long long)n_seqs * a.heads * ((col_warps + warps - 1) / warps) > 148) warps *= 2;
+    warps = min(warps, col_warps);
+    const int bytes = walk_smem_floats<RG, Delta, Fixed>(a.dim, a.rank, 32 * warps) * (int)sizeof(float);
+    constexpr int kMostBytes = 200 * 1024;
+    if (bytes > kMostBytes) return cudaErrorInvalidValue;
+    const cudaError_t e = allow_dynamic_smem(scan_walk_kernel<T, RG, Delta, Fixed>, kMostBytes, done);
+    if (e != cudaSuccess) return e;
+    return launch(scan_walk_kernel<T, RG, Delta, Fixed>, dim3(n_seqs, a.heads, (col_warps + warps - 1) / warps), 32 * warps + kWalkStagers, bytes,
+                  stream, a);
+}
+
+}  // namespace
+
+}  // namespace vtb
