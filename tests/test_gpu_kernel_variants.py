@@ -116,3 +116,29 @@ def test_walks_along_portions_equal_the_token_by_token_kernel(dim, v_dim, heads,
         for a, b in ((got, ref), (last, ref_last)):
             assert float((a - b).abs().max()) <= 2e-5 * max(1.0, float(b.abs().max())), name
         assert torch.equal(last[n:], state[n:])            # a row of no sequence of the step
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("n,k", [(16, 8), (48, 248), (1152, 896), (9728, 264), (896, 4864), (160, 2056)])
+def test_products_of_few_rows(m, n, k):
+    """bfloat16 in, 32-bit sums: every epilogue against float64."""
+    o = ops()
+    assert o.backend().gemm_tc_shares(m, n, k) == (4 if k >= 2048 and n <= 4096 else 1)      # (of the tcgen05 kernel: more)
+    g = torch.Generator(device=DEV).manual_seed(m * n + k)
+    x = torch.randn((m, k), generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn((n, k), generator=g, device=DEV) * k ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(n, generator=g, device=DEV)
+    ref = x.cpu().double() @ w.cpu().double().T
+    wide = o.linear(x, w, bias, torch.full((m, n), float("nan"), device=DEV))
+    assert float((wide.cpu().double() - ref - bias.cpu()).abs().max()) <= 2e-5
+    got = o.linear(x, w, None, torch.full((m, n), float("nan"), device=DEV, dtype=torch.bfloat16))
+    assert float(((got.cpu().double() - ref).abs() / (1 + ref.abs())).max()) <= 2.0 ** -8
+    share = o.linear_to_stream(x, w, bias)
+    assert float((share.dense().cpu().double() - ref - bias.cpu()).abs().max()) <= 2e-5
+    gate, up = ref.view(m, n // 16, 2, 8)[:, :, 0].reshape(m, -1), ref.view(m, n // 16, 2, 8)[:, :, 1].reshape(m, -1)
+    act = o.linear_silu_mul(x, w, torch.full((m, n // 2), float("nan"), device=DEV, dtype=torch.bfloat16))
+    want = gate / (1 + torch.exp(-gate)) * up
+    assert float(((act.cpu().double() - want).abs() / (1 + want.abs())).max()) <= 2.0 ** -8
+    sq = o.linear_relu_square(x, w, torch.full((m, n), float("nan"), device=DEV, dtype=torch.bfloat16))
+    want = ref.clamp(min=0) ** 2
+    assert float(((sq.cpu().double() - want).abs() / (1 + want)).max()) <= 2.0 ** -7

@@ -32,6 +32,7 @@ SOURCES = [
     "gemm_skinny.cu",
     "gemm_tc.cu",
     "gemm_tc_pair.cu",
+    "gemm_few.cu",
     "attention_noalloc.cu",
     "sampling.cu",
     "recurrent.cu",

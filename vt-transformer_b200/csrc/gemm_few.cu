@@ -1,0 +1,194 @@
+// out[M, N] = x[M, K] w[N, K]^T for up to eight rows of x in bfloat16 and matrices of a few megabytes, without tensor cores.
+//
+// Such a product is bound by neither bytes nor arithmetic but by the chain from one kernel to the next: in a decode step of a
+// small model a product has 1.6 to 17 MB to read (0.3 to 3 us at the copy bandwidth) and the tcgen05 kernel needs 5 us and more
+// for it (barriers, tensor memory, tensor maps, a ring that fills, an accumulator that is read back), and, holding all of an
+// SM's shared memory, cannot begin before the kernel in front has left.  Here a warp takes R rows of w whole; a lane has
+// 8 consecutive k of every 256, its numbers of w come straight into registers (the first DEPTH chunks before the dependency
+// wait: weights are no kernel's result, and with neither shared memory nor tensor memory to wait for the CTAs stand beside the
+// kernel in front), x comes through L1, products are added in 32-bit, two at a time (fma.rn.f32x2), and the lanes' sums
+// meet by shuffles.  Long rows are cut over KS warps of the CTA, whose sums are added in the order of the warps (or left
+// unadded as shares, for the norm that adds them while it reads).
+//
+// Measured on a B200: the decode step of one request at 0.5B sizes (24 layers) 910 us with the tcgen05 kernel, 614 with this one; 8 rows by
+// matrices of 1024 to 4096 x 1024 inside a step 9.2 and 6.5 us each.  The bound of 24 MB: matrices that take longer to stream than to reach
+// leave this kernel no advantage (7B sizes, 26 to 270 MB, stay with the other one).
+#include "common.cuh"
+#include "kernels.h"
+#include "launch.cuh"
+
+namespace vtb {
+
+namespace {
+
+constexpr int kFewWarps = 8;
+
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The two bfloat16 numbers of a word as a pair of floats.
+__device__ __forceinline__ unsigned long long widen(uint32_t u) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(u << 16), "r"(u & 0xffff0000u));
+    return r;
+}
+
+__device__ __forceinline__ uint4 load_once(const __nv_bfloat16* p) {      // (read by one warp: not kept in L1)
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
+// MT rows of x (at least m), R rows of w a warp, KS warps a row.  EPI as in gemm_epilogue.cuh (2: KS shares of k); with EPI 1
+// the two rows are the gate and the up of one feature.
+template <int MT, int R, int KS, int DEPTH, int EPI, typename TOut>
+__global__ void __launch_bounds__(32 * kFewWarps)
+gemm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias, TOut* __restrict__ out,
+                int m, int n, int k) {
+    static_assert(EPI != 1 || R == 2, "a feature's gate and up");
+    constexpr int V = R * MT;                     // a warp's sums
+    static_assert((V & (V - 1)) == 0 && V <= 32, "halved from round to round");
+    constexpr bool MEET = KS > 1 && EPI != 2;
+    __shared__ float part[MEET ? kFewWarps : 1][V];
+    pdl_launch();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int unit = (blockIdx.x * kFewWarps + warp) / KS, slice = KS > 1 ? warp % KS : 0;
+    const int units = EPI == 1 ? n / 2 : (n + R - 1) / R;
+    const bool live = unit < units;
+    auto row_of = [&](int r) { return EPI == 1 ? (unit >> 3) * 16 + (unit & 7) + 8 * r : min(unit * R + r, n - 1); };
+    const int chunks = (k + 255) / 256;
+    uint4 wv[DEPTH][R];
+    const __nv_bfloat16* wp[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) wp[r] = w + (live ? (size_t)row_of(r) * k : 0);
+    auto fetch = [&](int chunk, uint4 (&v)[R]) {
+        const int at = chunk * 256 + lane * 8;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = live && at < k ? load_once(wp[r] + at) : make_uint4(0u, 0u, 0u, 0u);
+    };
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) fetch(slice + d * KS, wv[d]);
+    pdl_wait();
+    unsigned long long acc[R][MT];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < MT; ++i) acc[r][i] = 0ull;
+    for (int base = slice; base < chunks; base += DEPTH * KS) {
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+            const int chunk = base + d * KS, at = chunk * 256 + lane * 8;
+            if (chunk >= chunks) break;
+            unsigned long long wide[R][4];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                wide[r][0] = widen(wv[d][r].x);
+                wide[r][1] = widen(wv[d][r].y);
+                wide[r][2] = widen(wv[d][r].z);
+                wide[r][3] = widen(wv[d][r].w);
+            }
+            fetch(chunk + DEPTH * KS, wv[d]);
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                const uint4 u = at < k ? *reinterpret_cast<const uint4*>(x + (size_t)min(i, m - 1) * k + at) : make_uint4(0u, 0u, 0u, 0u);
+                const unsigned long long xs[4] = {widen(u.x), widen(u.y), widen(u.z), widen(u.w)};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) acc[r][i] = fma_pair(wide[r][e], xs[e], acc[r][i]);
+            }
+        }
+    }
+    // the lanes' sums: each round halves the sums that a lane still has, then the lanes that hold the same one add up
+    float s[V];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(acc[r][i]));
+            s[r * MT + i] = lo + hi;
+        }
+    int mine = 0;                                 // the sum that this lane ends up with: row mine / MT of w, row mine % MT of x
+#pragma unroll
+    for (int o = 16, left = V; o > 0; o >>= 1) {
+        if (left > 1) {
+            left >>= 1;
+            const bool upper = lane & o;
+            mine += upper ? left : 0;
+#pragma unroll
+            for (int c = 0; c < left; ++c) {
+                const float give = upper ? s[c] : s[c + left], keep = upper ? s[c + left] : s[c];
+                s[c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        } else {
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+        }
+    }
+    float v = s[0];
+    if (MEET) {
+        if ((lane & (32 / V - 1)) == 0) part[warp][mine] = v;
+        __syncthreads();
+        if (slice != 0) return;
+        v = part[warp][mine];
+#pragma unroll
+        for (int q = 1; q < KS; ++q) v += part[warp + q][mine];
+    }
+    const int r = mine / MT, i = mine % MT;
+    const bool one = live && (lane & (32 / V - 1)) == 0 && i < m;      // of the lanes that hold the same sum
+    if (EPI == 1) {
+        const float up = __shfl_xor_sync(0xffffffffu, v, 16);         // (the first round parted the gate's sums from the up's)
+        if (one && r == 0) out[(size_t)i * (n / 2) + unit] = from_float<TOut>(v / (1.f + expf(-v)) * up);
+        return;
+    }
+    const int col = unit * R + r;
+    if (!one || col >= n) return;
+    if (EPI == 3) v = v > 0.f ? v * v : 0.f;
+    out[((size_t)(EPI == 2 ? slice * m : 0) + i) * n + col] = from_float<TOut>(v + (bias && (EPI != 2 || slice == 0) ? bias[col] : 0.f));
+}
+
+// rows that are long for their number are cut over four warps (fewer warps than the SMs hold would stream them alone)
+int few_shares(int n, int k) { return k >= 2048 && n <= 4096 ? 4 : 1; }
+
+template <int MT, int EPI, typename TOut>
+cudaError_t launch_few_rows(const __nv_bfloat16* x, const __nv_bfloat16* w, const float* bias, TOut* out, int m, int n, int k, cudaStream_t stream) {
+    if constexpr (EPI == 1) {
+        return launch(gemm_few_kernel<MT, 2, 1, 4, EPI, TOut>, (n / 2 + kFewWarps - 1) / kFewWarps, 32 * kFewWarps, 0, stream, x, w, bias, out, m, n, k);
+    } else {
+        if (few_shares(n, k) > 1)
+            return launch(gemm_few_kernel<MT, 1, 4, 4, EPI, TOut>, (n * 4 + kFewWarps - 1) / kFewWarps, 32 * kFewWarps, 0, stream, x, w, bias, out, m, n, k);
+        if (n >= 4 * kFewWarps * 148)
+            return launch(gemm_few_kernel<MT, (MT == 8 ? 2 : 4), 1, 4, EPI, TOut>, ((n + (MT == 8 ? 1 : 3)) / (MT == 8 ? 2 : 4) + kFewWarps - 1) / kFewWarps,
+                          32 * kFewWarps, 0, stream, x, w, bias, out, m, n, k);
+        return launch(gemm_few_kernel<MT, 1, 1, 4, EPI, TOut>, (n + kFewWarps - 1) / kFewWarps, 32 * kFewWarps, 0, stream, x, w, bias, out, m, n, k);
+    }
+}
+
+template <int EPI, typename TOut>
+cudaError_t launch_few(const void* x, const void* w, const float* bias, TOut* out, int m, int n, int k, cudaStream_t stream) {
+    const __nv_bfloat16 *xb = (const __nv_bfloat16*)x, *wb = (const __nv_bfloat16*)w;
+    if (m == 1) return launch_few_rows<1, EPI, TOut>(xb, wb, bias, out, m, n, k, stream);
+    if (m == 2) return launch_few_rows<2, EPI, TOut>(xb, wb, bias, out, m, n, k, stream);
+    if (m <= 4) return launch_few_rows<4, EPI, TOut>(xb, wb, bias, out, m, n, k, stream);
+    return launch_few_rows<8, EPI, TOut>(xb, wb, bias, out, m, n, k, stream);
+}
+
+}  // namespace
+
+bool gemm_few_takes(int m, int n, int k) { return m >= 1 && m <= 8 && k % 8 == 0 && 2LL * n * k <= 24LL << 20; }
+
+int gemm_few_shares(int n, int k) { return few_shares(n, k); }
+
+cudaError_t launch_gemm_few(int out_dtype, const void* x, const void* w, const float* bias, void* out, int m, int n, int k, int epilogue,
+                            cudaStream_t stream) {
+    if (epilogue == 1) return launch_few<1, __nv_bfloat16>(x, w, nullptr, (__nv_bfloat16*)out, m, n, k, stream);
+    if (epilogue == 3) return launch_few<3, __nv_bfloat16>(x, w, nullptr, (__nv_bfloat16*)out, m, n, k, stream);
+    if (epilogue == 2) return launch_few<2, float>(x, w, bias, (float*)out, m, n, k, stream);
+    if (out_dtype == kBF16) return launch_few<0, __nv_bfloat16>(x, w, bias, (__nv_bfloat16*)out, m, n, k, stream);
+    return launch_few<0, float>(x, w, bias, (float*)out, m, n, k, stream);
+}
+
+}  // namespace vtb
