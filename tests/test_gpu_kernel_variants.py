@@ -90,7 +90,7 @@ def walked(o, name, y, state, ctx, v_dim, heads, walk, call):
 @pytest.mark.parametrize("dim,v_dim,heads", [(34, 32, 3), (64, 64, 2), (64, 136, 5), (66, 40, 2), (128, 256, 2), (120, 90, 40)])
 @pytest.mark.parametrize("lens", [[1, 16, 47], [17, 33, 15, 100]])
 def test_walks_along_portions_equal_the_token_by_token_kernel(dim, v_dim, heads, lens):
-    """Gated linear attention, delta rule and retention in bfloat16 portions: results and last states of both kernels, whose sums differ
+    """Gated linear attention and the delta rule in bfloat16 portions: results and last states of both kernels, whose sums differ
     in their order alone (32-bit sums of up to 128 terms, and what a recurrence of 100 tokens makes of them)."""
     o, rank = ops(), 16
     g = torch.Generator().manual_seed(dim + v_dim)
@@ -102,12 +102,9 @@ def test_walks_along_portions_equal_the_token_by_token_kernel(dim, v_dim, heads,
     v_col = low_col + rank
     y = (rnd(T, v_col + heads * max(v_dim, dim) + (heads * max(v_dim, dim)) % 2) * 0.5).to(torch.bfloat16)
     w2, b2, ab = rnd(heads * dim, rank) * 0.3, rnd(heads * dim), rnd(heads * dim)
-    decay = torch.linspace(0.5, 0.999, heads).to(DEV)
-    freq = torch.linspace(1.0, 0.01, dim // 4).to(DEV)
     cases = {
         "gla": (v_dim, lambda st, out: o.gla_scan(y, q_col, k_col, v_col, low_col, w2, b2, 1 / 16, dim ** -0.5, st, ctx, out, heads, dim, v_dim)),
         "delta": (dim, lambda st, out: o.delta_scan(y, q_col, k_col, v_col, a_col, low_col, w2, b2, ab, math.exp(-0.5), 1e-6, st, ctx, out, heads, dim)),
-        "retention": (v_dim, lambda st, out: o.retention_scan(y, q_col, k_col, v_col, decay, dim ** -0.5, freq, st, ctx, out, heads, dim, v_dim, act=True)),
     }
     for name, (cols, call) in cases.items():
         state = rnd(rows, heads, dim, cols)

@@ -382,9 +382,9 @@ namespace {
 
 template <typename T, bool Delta, bool Fixed = false>
 cudaError_t launch_scan_t(ScanArgs a, int n_seqs, cudaStream_t stream) {
-    if constexpr (sizeof(T) == 2) {
-        if (walk_takes(a) && walk_smem_floats<8, Delta, Fixed>(a.dim, a.rank, 128) * 4 <= 200 * 1024)
-            return a.dim <= 64 ? launch_scan_walk<T, 4, Delta, Fixed>(a, n_seqs, stream) : launch_scan_walk<T, 8, Delta, Fixed>(a, n_seqs, stream);
+    if constexpr (sizeof(T) == 2 && !Fixed) {
+        if (walk_takes(a) && walk_smem_floats<8, Delta>(a.dim, a.rank, 128) * 4 <= 200 * 1024)
+            return a.dim <= 64 ? launch_scan_walk<T, 4, Delta>(a, n_seqs, stream) : launch_scan_walk<T, 8, Delta>(a, n_seqs, stream);
     }
     // Rows a thread: 16 where that makes at most 8 groups of warps a column, else 32, 64, 128.  Few rows a thread make
     // the walk along the tokens short (a token costs a thread rows / 4 steps of loads and multiply-adds, whatever the

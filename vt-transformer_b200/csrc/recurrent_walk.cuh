@@ -1,16 +1,15 @@
-// The recurrences of recurrent.cu along a portion of a prompt in bfloat16 steps, for keys of 33 to 128 numbers.
+// The gated recurrences of recurrent.cu along a portion of a prompt in bfloat16 steps, for keys of 33 to 128 numbers.
 //
 // What bounds the walk is a sequence's own chain: a token's multiply-adds, the numbers that shared memory delivers for
 // them (a warp's 16-byte load takes four cycles whatever its lanes share) and the meeting of the threads that hold a
 // column.  A thread here holds 16 rows of CPT columns, so that a number of q, k or the decay that it loads serves CPT
 // multiply-adds, and the RG threads that share a column are neighbours in one warp: they meet by shuffles, no barrier
-// stands inside a token.  Four more warps stage the next 16 tokens (loads, gates, unit keys, rotation) while the others
+// stands inside a token.  Four more warps stage the next 16 tokens (loads, gates, unit keys) while the others
 // walk.  State, gates and sums are 32-bit as in scan_kernel; only the order of the sums over a column differs, which is why
 // a 32-bit step, whose tokens must not depend on what else is in the step, stays with scan_kernel.
 //
-// Measured on a B200, us, scan_kernel's walk and this one: 4 sequences of up to 1,500 tokens, 8 heads: gated linear attention of
-// 64 x 128 1,119 and 722, delta rule of 64 x 64 1,755 and 960; retention of 16 heads of 128 x 256 over 4,096 tokens in segments 1,471 and
-// 580.  Four columns a thread for keys of more than 64 numbers (twice the warps, half the registers) were slower: 634.
+// Measured on a B200, us, scan_kernel's walk and this one: 4 sequences of up to 1,500 tokens, 8 heads: gated linear
+// attention of 64 x 128 1,119 and 722, delta rule of 64 x 64 1,755 and 960.  Retention (recurrent.cu) stays with scan_kernel.
 #pragma once
 
 namespace vtb {
@@ -44,19 +43,19 @@ __device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
     return r;
 }
 
-// Numbers of a staged token: q, k, then the decay (not with Fixed), then b = a u and u (Delta); the values lie apart.
-template <bool Delta, bool Fixed> __host__ __device__ constexpr int walk_vectors() { return Delta ? 5 : (Fixed ? 2 : 3); }
+// Numbers of a staged token: q, k, then the decay, then b = a u and u (Delta); the values lie apart.
+template <bool Delta> __host__ __device__ constexpr int walk_vectors() { return Delta ? 5 : 3; }
 
-template <int RG, bool Delta, bool Fixed>
+template <int RG, bool Delta>
 __host__ __device__ inline int walk_smem_floats(int dim, int rank, int cols) {
-    return ((dim * rank + 3) & ~3) + ((kWalkTokens * rank + 3) & ~3) + 2 * kWalkTokens * (walk_vectors<Delta, Fixed>() * 16 * RG + cols);
+    return ((dim * rank + 3) & ~3) + ((kWalkTokens * rank + 3) & ~3) + 2 * kWalkTokens * (walk_vectors<Delta>() * 16 * RG + cols);
 }
 
 // RG: the threads that share a column (16 rows each); they hold CPT = RG columns each, so a warp has 32.
-template <typename T, int RG, bool Delta, bool Fixed>
+template <typename T, int RG, bool Delta>
 __global__ void __launch_bounds__(kWalkStagers + 32 * kWalkWarps, 1)
 scan_walk_kernel(const ScanArgs a) {
-    constexpr int CPT = RG, DP = 16 * RG, TB = kWalkTokens, VEC = walk_vectors<Delta, Fixed>();
+    constexpr int CPT = RG, DP = 16 * RG, TB = kWalkTokens, VEC = walk_vectors<Delta>();
     constexpr int D_AT = 2, B_AT = 3, U_AT = 4;
     extern __shared__ __align__(16) float smem[];
     pdl_launch();
@@ -74,13 +73,11 @@ scan_walk_kernel(const ScanArgs a) {
     const int t0 = a.cu_q[seq], t1 = a.cu_q[seq + 1];
     if (t1 <= t0) return;                                   // a sequence without tokens in this step (padding): its state stays
     const int row = a.rows[seq];
-    const bool later = Fixed && row < 0 && a.ends != nullptr;      // a later segment of a walk that was cut
-    if (later ? (-row - 1 >= a.end_rows) : (row < 0 || row >= a.state_rows)) {
+    if (row < 0 || row >= a.state_rows) {
         if (tid == 0) set_status(a.status, kStatusBadRow, row);
         return;
     }
-    float* sp = later ? a.ends + (((size_t)(-row - 1) * a.heads + h) * dim) * v_dim
-                      : a.state + (((size_t)row * a.heads + h) * dim) * v_dim;
+    float* sp = a.state + (((size_t)row * a.heads + h) * dim) * v_dim;
     const T* y = reinterpret_cast<const T*>(a.y);
     const int batches = (t1 - t0 + TB - 1) / TB;
     const int st = tid - walkers;                           // a staging thread's number (negative: it walks)
@@ -95,11 +92,10 @@ scan_walk_kernel(const ScanArgs a) {
 #pragma unroll
             for (int c = 0; c < CPT; ++c) {
                 const int r = 4 * (rg + RG * (i >> 1)) + 2 * (i & 1), j = col0 + wc + c;
-                const bool in = !later && j < v_dim;
+                const bool in = j < v_dim;
                 S[i][c] = pair_of(in && r < dim ? sp[(size_t)r * v_dim + j] : 0.f, in && r + 1 < dim ? sp[(size_t)(r + 1) * v_dim + j] : 0.f);
             }
     }
-    const float decay = Fixed ? a.bias2[h] : 0.f;
 
     // ---- staging ----------------------------------------------------------------------------------------------
     // two neighbouring numbers of a token at a time: q, k and (Delta) the removal rate, each DP wide, the gate's input, the values
@@ -114,11 +110,10 @@ scan_walk_kernel(const ScanArgs a) {
             int from = -1, step;
             float* dst;
             float times = 1.f;
-            bool act = Fixed && a.act != 0;
             if (r < kRead * DP) {
                 const int which = r / DP, i = r - which * DP;
                 if (i < dim) from = (which == 0 ? a.q_col : (which == 1 ? a.k_col : a.a_col)) + h * dim + i;
-                if (!Delta && which == (Fixed ? 1 : 0)) times = a.c2;
+                if (!Delta && which == 0) times = a.c2;
                 dst = to + (which == 2 ? B_AT : which) * DP + i;
                 step = VEC * DP;
             } else if (r < kRead * DP + cols) {
@@ -131,7 +126,6 @@ scan_walk_kernel(const ScanArgs a) {
                 from = a.low_col + i;
                 dst = low + i;
                 step = rank;
-                act = false;
             }
             const bool is_low = r >= kRead * DP + cols;
             const T* src = y + (size_t)first * a.stride + (from < 0 ? 0 : from);
@@ -145,10 +139,6 @@ scan_walk_kernel(const ScanArgs a) {
             for (int t = 0; t < TB; ++t) {
                 if (t >= n) break;
                 float2 v = val[t];
-                if (act) {
-                    v.x = v.x / (1.f + expf(-v.x));
-                    v.y = v.y / (1.f + expf(-v.y));
-                }
                 v.x *= times;
                 v.y *= times;
                 if (Delta && is_low) {
@@ -159,41 +149,24 @@ scan_walk_kernel(const ScanArgs a) {
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kWalkStagers) : "memory");
-        if (Fixed) {
-            // the rotation of q and k: a thread turns both members of a pair, so nothing else touches them meanwhile
-            const int half = a.half;
-            for (int e = st; e < n * half; e += kWalkStagers) {
-                const int t = e / half, i = e % half;
-                float sn, cs;
-                sincosf((float)a.positions[first + t] * a.freq[i], &sn, &cs);
-                float* qv = to + t * VEC * DP;
-                float* kv = qv + DP;
-                const float qa = qv[i], qb = qv[i + half], ka = kv[i], kb = kv[i + half];
-                qv[i] = qa * cs - qb * sn;
-                qv[i + half] = qb * cs + qa * sn;
-                kv[i] = ka * cs - kb * sn;
-                kv[i + half] = kb * cs + ka * sn;
-            }
-        } else {
-            for (int e = st; e < n * DP; e += kWalkStagers) {
-                const int t = e / DP, i = e % DP;
-                float d = 0.f;
-                if (i < dim) {
-                    const int ch = h * dim + i;
-                    float z = a.bias2[ch];
-                    const float* wr = w2s + i * rank;
-                    const float* lr = low + t * rank;
-                    for (int r = 0; r < rank; ++r) z = fmaf(wr[r], lr[r], z);
-                    if (Delta) {
-                        d = expf(-a.c1 * sigmoid(z));
-                        float* b = to + t * VEC * DP + B_AT * DP + i;
-                        *b = sigmoid(*b + a.a_bias[ch]);
-                    } else {
-                        d = expf(a.c1 * log_sigmoid(z));
-                    }
+        for (int e = st; e < n * DP; e += kWalkStagers) {
+            const int t = e / DP, i = e % DP;
+            float d = 0.f;
+            if (i < dim) {
+                const int ch = h * dim + i;
+                float z = a.bias2[ch];
+                const float* wr = w2s + i * rank;
+                const float* lr = low + t * rank;
+                for (int r = 0; r < rank; ++r) z = fmaf(wr[r], lr[r], z);
+                if (Delta) {
+                    d = expf(-a.c1 * sigmoid(z));
+                    float* b = to + t * VEC * DP + B_AT * DP + i;
+                    *b = sigmoid(*b + a.a_bias[ch]);
+                } else {
+                    d = expf(a.c1 * log_sigmoid(z));
                 }
-                to[t * VEC * DP + D_AT * DP + i] = d;
             }
+            to[t * VEC * DP + D_AT * DP + i] = d;
         }
         if (Delta) {
             asm volatile("bar.sync 1, %0;" ::"n"(kWalkStagers) : "memory");
@@ -219,7 +192,6 @@ scan_walk_kernel(const ScanArgs a) {
         const float* vat = values + (batch & 1) * TB * cols + wc;
         const int j = col0 + wc + rg;                       // the column whose sum this lane ends up with
         float* o = a.out + (size_t)first * a.heads * v_dim + h * v_dim + j;
-        const Pair fixed = pair_of(decay, decay);
         for (int t = 0; t < n; ++t, at += VEC * DP, vat += cols, o += a.heads * v_dim) {
             Pair v[CPT], acc[CPT], gone[CPT];
 #pragma unroll
@@ -255,8 +227,8 @@ scan_walk_kernel(const ScanArgs a) {
             for (int i = 0; i < 4; ++i) {
                 const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(at + 4 * RG * i);
                 const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(at + DP + 4 * RG * i);
-                ulonglong2 d = make_ulonglong2(fixed.v, fixed.v), b = make_ulonglong2(0ull, 0ull);
-                if (!Fixed) d = *reinterpret_cast<const ulonglong2*>(at + D_AT * DP + 4 * RG * i);
+                const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(at + D_AT * DP + 4 * RG * i);
+                ulonglong2 b = make_ulonglong2(0ull, 0ull);
                 if (Delta) b = *reinterpret_cast<const ulonglong2*>(at + B_AT * DP + 4 * RG * i);
                 const Pair qs[2] = {{q.x}, {q.y}}, ks[2] = {{k.x}, {k.y}}, ds[2] = {{d.x}, {d.y}}, bs[2] = {{b.x}, {b.y}};
 #pragma unroll
@@ -314,7 +286,7 @@ inline bool walk_takes(const ScanArgs& a) {
            ((a.q_col | a.k_col | a.v_col | a.a_col | a.low_col) & 1) == 0 && ((uintptr_t)a.y & 3) == 0;
 }
 
-template <typename T, int RG, bool Delta, bool Fixed>
+template <typename T, int RG, bool Delta>
 cudaError_t launch_scan_walk(const ScanArgs& a, int n_seqs, cudaStream_t stream) {
     static std::atomic<unsigned long long> done{0};
     // warps of 32 columns a CTA: as few as keep the CTAs within one round (each stages its tokens for itself)
@@ -322,12 +294,12 @@ cudaError_t launch_scan_walk(const ScanArgs& a, int n_seqs, cudaStream_t stream)
     int warps = 1;
     while (warps < kWalkWarps && (long long)n_seqs * a.heads * ((col_warps + warps - 1) / warps) > 148) warps *= 2;
     warps = min(warps, col_warps);
-    const int bytes = walk_smem_floats<RG, Delta, Fixed>(a.dim, a.rank, 32 * warps) * (int)sizeof(float);
+    const int bytes = walk_smem_floats<RG, Delta>(a.dim, a.rank, 32 * warps) * (int)sizeof(float);
     constexpr int kMostBytes = 200 * 1024;
     if (bytes > kMostBytes) return cudaErrorInvalidValue;
-    const cudaError_t e = allow_dynamic_smem(scan_walk_kernel<T, RG, Delta, Fixed>, kMostBytes, done);
+    const cudaError_t e = allow_dynamic_smem(scan_walk_kernel<T, RG, Delta>, kMostBytes, done);
     if (e != cudaSuccess) return e;
-    return launch(scan_walk_kernel<T, RG, Delta, Fixed>, dim3(n_seqs, a.heads, (col_warps + warps - 1) / warps), 32 * warps + kWalkStagers, bytes,
+    return launch(scan_walk_kernel<T, RG, Delta>, dim3(n_seqs, a.heads, (col_warps + warps - 1) / warps), 32 * warps + kWalkStagers, bytes,
                   stream, a);
 }
 
