@@ -139,3 +139,34 @@ def test_products_of_few_rows(m, n, k):
     sq = o.linear_relu_square(x, w, torch.full((m, n), float("nan"), device=DEV, dtype=torch.bfloat16))
     want = ref.clamp(min=0) ** 2
     assert float(((sq.cpu().double() - want).abs() / (1 + want)).max()) <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("heads,kv_heads,d,page,window,sink,cap", [(14, 2, 64, 64, None, False, None), (28, 4, 128, 64, None, True, None),
+                                                                   (8, 2, 128, 16, 3000, False, 20.0), (16, 1, 64, 32, None, True, 30.0)])
+@pytest.mark.parametrize("lens,starts", [([130, 70], [5000, 2001]), ([1, 1, 1, 90], [40, 900, 3, 6111])])
+def test_attention_tiles_in_pieces_equal_whole_tiles(monkeypatch, heads, kv_heads, d, page, window, sink, cap, lens, starts):
+    """Few tiles over long contexts: the pieces put together equal the whole tiles up to the rounding of P (2^-9 of values of unit size)
+    and of the result; twice, since the counters have to be zero again."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(d + sum(lens))
+    totals = [a + b for a, b in zip(lens, starts)]
+    k, v = (torch.randn((sum(totals), kv_heads, d), generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    kc, vc, table = paged_cache(k, v, totals, page, sum(-(-n // page) for n in totals) + 3, torch.bfloat16, seed=4)
+    T = sum(lens)
+    qkv = (torch.randn((T, (heads + 2 * kv_heads) * d), generator=g, device=DEV) * 2).to(torch.bfloat16)
+    sinks = torch.linspace(-1, 3, heads).to(DEV) if sink else None
+    ctx = helpers.step_context(lens, starts, DEV)
+    status = torch.zeros(2, dtype=torch.int32, device=DEV)
+
+    def run():
+        out = torch.full((T, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+        o.paged_attention(qkv, out, kc, vc, ctx, table, heads, kv_heads, d, window, 1 / math.sqrt(d), status=status, sinks=sinks, softcap=cap)
+        return out.float()
+    first, again = run(), run()
+    cut = [p for key, p in ctx.extras.items() if key[0] == "attention_pieces"]
+    assert len(cut) == 1 and cut[0] and int(cut[0][0][:, 7].max()) > 1 and int(cut[0][1].abs().sum()) == 0
+    assert torch.equal(first, again)
+    monkeypatch.setattr(o, "_attention_pieces", lambda *a: {})
+    whole = run()
+    assert status.tolist() == [0, 0]
+    assert float((first - whole).abs().max()) <= 2.0 ** -7 * max(1.0, float(whole.abs().max()))

@@ -24,6 +24,11 @@
 // below 2^8, exact in the 32-bit sum and with the same relative rounding in bfloat16); raising it means
 // multiplying O in tensor memory by the correction, which then happens in few blocks only.
 //
+// A tile's blocks may be cut into pieces, a CTA each, where whole tiles would leave SMs idle (few tiles over long contexts, a last round
+// that is nearly empty; the caller decides, see attention_pieces in binding.cpp).  A piece leaves its rows' unnormalised results with
+// their maxima and sums in scratch memory, and the CTA of a tile that arrives last (a counter a tile, left zero) puts the pieces
+// together in their order; no CTA waits for another.
+//
 // Warp 0 loads (one thread), warp 1 issues the MMAs (one thread), warps 2..5 and 6..9 are the two groups.
 // Every wait on a barrier is bounded; a wait that runs out sets the status word and the CTA winds down.
 #include <cuda.h>
@@ -61,6 +66,12 @@ struct AttnTcParams {
     int cache_rows;          // pages * kv_heads * page_size: a row index beyond it makes TMA fill zeros
     int* status;
     const float* sinks;      // [heads] or null: one more term exp(sinks[head]) in a row's denominator, without a key or a value
+    // pieces of tiles (null: a CTA a tile): two int4 each, (sequence, first token, KV head, tile) and (first block, blocks, the piece's
+    // number among its tile's, how many the tile has); scratch [pieces][D / 4][128 rows][4], ml [pieces][128 rows][maximum, sum]
+    const int4* pieces;
+    float* part_o;
+    float2* part_ml;
+    int* counters;           // [tiles]
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -141,7 +152,7 @@ __device__ __forceinline__ void write_p_half(const uint32_t (&raw)[TK], uint32_t
     }
 }
 
-template <int D, bool CAP>
+template <int D, bool CAP, bool PIECES>
 __global__ void __launch_bounds__(ATC_THREADS)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     const AttnTcParams p) {
@@ -163,8 +174,19 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // what the step's own inputs say about this tile (they are there before the step's first kernel starts)
-    const int kvh = blockIdx.y;
-    const int2 tl = p.tiles[blockIdx.x];
+    int kvh = blockIdx.y;
+    int2 tl;
+    int4 piece = make_int4(0, 1 << 30, 0, 1);            // (first block, blocks, which of the tile's pieces, how many)
+    int tile_id = 0;
+    if constexpr (PIECES) {
+        const int4 at = p.pieces[2 * blockIdx.x];
+        piece = p.pieces[2 * blockIdx.x + 1];
+        tl = make_int2(at.x, at.y);
+        kvh = at.z;
+        tile_id = at.w;
+    } else {
+        tl = p.tiles[blockIdx.x];
+    }
     const int seq = tl.x, tok0 = tl.y;
     const int q_begin = p.cu_q[seq];
     const int q_len = p.cu_q[seq + 1] - q_begin;
@@ -174,9 +196,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int start = p.q_start[seq];
     const int pos_lo = start + tok0, pos_hi = pos_lo + max(1, ntok) - 1;
     int key_lo = first_visible_key(pos_lo, p.window, p.chunk);
-    key_lo = key_lo / TK * TK;
-    const int key_hi = pos_hi + 1;
-    const int nb = (ntok > 0) ? (key_hi - key_lo + TK - 1) / TK : 0;
+    key_lo = key_lo / TK * TK + (PIECES ? piece.x * TK : 0);
+    const int whole = (ntok > 0) ? (pos_hi + 1 - key_lo + TK - 1) / TK : 0;
+    const int nb = PIECES ? min(piece.y, whole) : whole;
+    const int key_hi = PIECES ? min(pos_hi + 1, key_lo + nb * TK) : pos_hi + 1;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&k_full[i], 1);
@@ -323,7 +346,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const uint32_t s_addr = tmem + lane_base + (uint32_t)(g * TK);
         const uint32_t o_addr = tmem + lane_base + (uint32_t)(2 * TK + g * D);
         float m = -INFINITY, l = 0.f;       // the maximum P is scaled by (in log2 units), and the sum at that scale
-        if (p.sinks != nullptr && g == 0 && valid) {
+        if (p.sinks != nullptr && g == 0 && valid && (!PIECES || piece.z == 0)) {
             // the sink is a first key without a value, in the group of the even blocks: its score is the scale to begin
             // with and it counts once in the sum
             m = p.sinks[head] * 1.4426950408889634f;
@@ -422,7 +445,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 const float w_mine = (m == -INFINITY) ? 0.f : ex2(m - m_all);
                 const float w_other = (m_other == -INFINITY) ? 0.f : ex2(m_other - m_all);
                 const float sum = l * w_mine + l_other * w_other;
-                const float inv = sum > 0.f ? 1.f / sum : 0.f;
+                const float inv = (PIECES && piece.w > 1) ? 1.f : (sum > 0.f ? 1.f / sum : 0.f);
                 const float w_even = (g == 0 ? w_mine : w_other) * inv, w_odd = (g == 0 ? w_other : w_mine) * inv;
                 __nv_bfloat16* dst = p.out + ((size_t)tok * p.heads + head) * D + g * (D / 2);
                 // the loads of tensor memory are warp-wide: rows without a query take part and store nothing
@@ -437,7 +460,18 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                         for (int i = 0; i < 32; ++i) odd[i] = 0u;
                     }
 #pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        if (!PIECES || piece.w == 1) break;
+                        float4 v;
+                        v.x = __uint_as_float(even[i]) * w_even + __uint_as_float(odd[i]) * w_odd;
+                        v.y = __uint_as_float(even[i + 1]) * w_even + __uint_as_float(odd[i + 1]) * w_odd;
+                        v.z = __uint_as_float(even[i + 2]) * w_even + __uint_as_float(odd[i + 2]) * w_odd;
+                        v.w = __uint_as_float(even[i + 3]) * w_even + __uint_as_float(odd[i + 3]) * w_odd;
+                        *reinterpret_cast<float4*>(p.part_o + (((size_t)blockIdx.x * (D / 4) + (g * (D / 2) + c0 + i) / 4) * 128 + r) * 4) = v;
+                    }
+#pragma unroll
                     for (int i = 0; i < 32; i += 8) {
+                        if (PIECES && piece.w > 1) break;
                         uint4 u4;
                         __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&u4);
 #pragma unroll
@@ -447,6 +481,54 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                                 __uint_as_float(even[i + 2 * e + 1]) * w_even + __uint_as_float(odd[i + 2 * e + 1]) * w_odd);
                         if (valid) *reinterpret_cast<uint4*>(dst + c0 + i) = u4;
                     }
+                }
+                if (PIECES && piece.w > 1 && g == 0) p.part_ml[(size_t)blockIdx.x * 128 + r] = make_float2(m_all, sum);
+            }
+        }
+    }
+    if (PIECES && piece.w > 1) {
+        // the tile's last piece to arrive puts all of them together (a piece that gave up arrives too: the counter has to come out even)
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int before = atomicAdd(p.counters + tile_id, 1);
+            *tmem_slot = before == piece.w - 1 ? 1u : 0u;
+            if (before == piece.w - 1) p.counters[tile_id] = 0;
+        }
+        __syncthreads();
+        if (*tmem_slot != 0u && warp >= 2) {
+            __threadfence();
+            const int g = (warp - 2) >> 2, r = (warp & 3) * 32 + lane;
+            const size_t first = blockIdx.x - piece.z;             // (a tile's pieces stand side by side)
+            float m_all = -INFINITY;
+            for (int i = 0; i < piece.w; ++i) m_all = fmaxf(m_all, __ldcg(&p.part_ml[(first + i) * 128 + r]).x);
+            float sum = 0.f;
+            for (int i = 0; i < piece.w; ++i) {
+                const float2 ml = __ldcg(&p.part_ml[(first + i) * 128 + r]);
+                if (ml.x != -INFINITY) sum += ml.y * ex2(ml.x - m_all);
+            }
+            const float inv = sum > 0.f ? 1.f / sum : 0.f;
+            if (r < rows_valid) {
+                const int tok = q_begin + tok0 + r / group, head = kvh * group + r % group;
+                __nv_bfloat16* dst = p.out + ((size_t)tok * p.heads + head) * D + g * (D / 2);
+#pragma unroll 1
+                for (int c = 0; c < D / 2; c += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+                    for (int i = 0; i < piece.w; ++i) {
+                        const float mi = __ldcg(&p.part_ml[(first + i) * 128 + r]).x;
+                        const float f = mi == -INFINITY ? 0.f : ex2(mi - m_all);
+                        const float4* at = reinterpret_cast<const float4*>(p.part_o + (((first + i) * (D / 4) + (g * (D / 2) + c) / 4) * 128 + r) * 4);
+                        const float4 a = __ldcg(at), b = __ldcg(at + 128);
+                        v[0] = fmaf(a.x, f, v[0]); v[1] = fmaf(a.y, f, v[1]); v[2] = fmaf(a.z, f, v[2]); v[3] = fmaf(a.w, f, v[3]);
+                        v[4] = fmaf(b.x, f, v[4]); v[5] = fmaf(b.y, f, v[5]); v[6] = fmaf(b.z, f, v[6]); v[7] = fmaf(b.w, f, v[7]);
+                    }
+                    uint4 u4;
+                    __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&u4);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) hp[e] = __floats2bfloat162_rn(v[2 * e] * inv, v[2 * e + 1] * inv);
+                    *reinterpret_cast<uint4*>(dst + c) = u4;
                 }
             }
         }
@@ -470,9 +552,10 @@ cudaError_t launch_attention_tc(const void* qkv, int qkv_stride, void* out, cons
                                 const int* cu_q, const int* q_start, const int* block_table, int table_stride,
                                 const int* tiles, int n_tiles, int n_pages, int heads, int kv_heads, int head_dim,
                                 int page_size, int window, float scale, int* status, cudaStream_t stream, int chunk,
-                                const float* sinks, float softcap) {
-    if (n_tiles == 0) return cudaSuccess;
-    if (!attention_tc_supports(head_dim, heads, kv_heads) || page_size % 16 != 0 || tiles == nullptr) return cudaErrorInvalidValue;
+                                const float* sinks, float softcap, const int* pieces, int n_pieces, float* part_o, float* part_ml, int* counters) {
+    if (n_tiles == 0 && n_pieces == 0) return cudaSuccess;
+    if (!attention_tc_supports(head_dim, heads, kv_heads) || page_size % 16 != 0 || (tiles == nullptr && pieces == nullptr)) return cudaErrorInvalidValue;
+    if (pieces != nullptr && (part_o == nullptr || part_ml == nullptr || counters == nullptr)) return cudaErrorInvalidValue;
     const long long cache_rows = (long long)n_pages * kv_heads * page_size;
     if (cache_rows >= (1LL << 31) - 256) return cudaErrorInvalidValue;
     CUtensorMap map_k, map_v;
@@ -501,17 +584,26 @@ cudaError_t launch_attention_tc(const void* qkv, int qkv_stride, void* out, cons
     p.run_keys = run_keys;
     p.status = status;
     p.sinks = sinks;
+    p.pieces = (const int4*)pieces;
+    p.part_o = part_o;
+    p.part_ml = (float2*)part_ml;
+    p.counters = counters;
     // Q, two stages of K and of V (HALVES halves of 16 KB each), barriers, the exchange; never so little that two CTAs
     // would fit an SM: each takes all of its tensor memory
     const int halves = head_dim / 64;
     const int smem = max((1 + 2 * 2) * halves * HALF_BYTES + 1024 + 256 + 2 * 128 * 2 * 4, 120 * 1024);
     const bool cap = softcap > 0.f;
-    auto kernel = head_dim == 128 ? (cap ? attention_tc_kernel<128, true> : attention_tc_kernel<128, false>)
-                                  : (cap ? attention_tc_kernel<64, true> : attention_tc_kernel<64, false>);
-    static std::atomic<unsigned long long> configured[4] = {{0}, {0}, {0}, {0}};
-    cudaError_t e = allow_dynamic_smem(kernel, smem, configured[2 * (halves - 1) + (cap ? 1 : 0)]);
+    const bool cut = pieces != nullptr;
+    auto pick = [&](auto whole, auto in_pieces) { return cut ? in_pieces : whole; };
+    auto kernel = head_dim == 128
+        ? (cap ? pick(attention_tc_kernel<128, true, false>, attention_tc_kernel<128, true, true>)
+               : pick(attention_tc_kernel<128, false, false>, attention_tc_kernel<128, false, true>))
+        : (cap ? pick(attention_tc_kernel<64, true, false>, attention_tc_kernel<64, true, true>)
+               : pick(attention_tc_kernel<64, false, false>, attention_tc_kernel<64, false, true>));
+    static std::atomic<unsigned long long> configured[8] = {{0}, {0}, {0}, {0}, {0}, {0}, {0}, {0}};
+    cudaError_t e = allow_dynamic_smem(kernel, smem, configured[4 * (halves - 1) + (cap ? 2 : 0) + (cut ? 1 : 0)]);
     if (e != cudaSuccess) return e;
-    return launch(kernel, dim3(n_tiles, kv_heads, 1), dim3(ATC_THREADS, 1, 1), smem, stream, map_k, map_v, p);
+    return launch(kernel, pieces != nullptr ? dim3(n_pieces, 1, 1) : dim3(n_tiles, kv_heads, 1), dim3(ATC_THREADS, 1, 1), smem, stream, map_k, map_v, p);
 }
 
 }  // namespace vtb

@@ -4,6 +4,13 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
+#include <cstring>
+#include <functional>
+#include <queue>
+#include <utility>
+#include <vector>
+
 #include "kernels.h"
 
 namespace {
@@ -1328,7 +1335,8 @@ bool attention_tc_supports(int64_t head_dim, int64_t heads, int64_t kv_heads) {
 void attention_tc(const Tensor& qkv, Tensor& out, const Tensor& k_cache, const Tensor& v_cache, const Tensor& cu_q,
                   const Tensor& q_start, const Tensor& block_table, const Tensor& tiles, int64_t heads, int64_t kv_heads,
                   int64_t head_dim, int64_t window, double scale, c10::optional<Tensor> status, int64_t chunk, c10::optional<Tensor> sinks,
-                  double softcap) {
+                  double softcap, c10::optional<Tensor> pieces, c10::optional<Tensor> part_o, c10::optional<Tensor> part_ml,
+                  c10::optional<Tensor> counters) {
     check_cuda(qkv, "qkv"); check_cuda(out, "out"); check_i32(cu_q, "cu_q"); check_i32(q_start, "q_start");
     check_i32(block_table, "block_table"); check_i32(tiles, "tiles");
     TORCH_CHECK(softcap >= 0.0, "attention_tc: softcap not negative");
@@ -1357,14 +1365,100 @@ void attention_tc(const Tensor& qkv, Tensor& out, const Tensor& k_cache, const T
         TORCH_CHECK(sinks->numel() == heads, "attention_tc: one sink a head");
         sinks_tc = sinks->data_ptr<float>();
     }
+    int n_pieces = 0;
+    if (pieces.has_value()) {
+        TORCH_CHECK(part_o.has_value() && part_ml.has_value() && counters.has_value(), "attention_tc: pieces of tiles need scratch and counters");
+        check_i32(*pieces, "pieces"); check_f32(*part_o, "part_o"); check_f32(*part_ml, "part_ml"); check_i32(*counters, "counters");
+        n_pieces = pieces->size(0);
+        TORCH_CHECK(pieces->dim() == 2 && pieces->size(1) == 8 && part_o->numel() >= (int64_t)n_pieces * 128 * head_dim &&
+                        part_ml->numel() >= (int64_t)n_pieces * 256 && counters->numel() >= tiles.size(0) * kv_heads,
+                    "attention_tc: pieces [n, 8], 128 * head_dim and 256 floats of scratch a piece, a counter a tile and KV head");
+    }
     c10::cuda::CUDAGuard guard(qkv.device());
     check_launch(vtb::launch_attention_tc(qkv.data_ptr(), qkv.size(1), out.data_ptr(), k_cache.data_ptr(),
                                           v_cache.data_ptr(), cu_q.data_ptr<int>(), q_start.data_ptr<int>(),
                                           block_table.data_ptr<int>(), block_table.size(1), tiles.data_ptr<int>(),
                                           tiles.size(0), k_cache.size(0), heads, kv_heads, head_dim, k_cache.size(2),
                                           window, (float)scale, status_ptr(status), stream_of(qkv), (int)chunk, sinks_tc,
-                                          (float)softcap),
+                                          (float)softcap, n_pieces ? pieces->data_ptr<int>() : nullptr, n_pieces,
+                                          n_pieces ? part_o->data_ptr<float>() : nullptr, n_pieces ? part_ml->data_ptr<float>() : nullptr,
+                                          n_pieces ? counters->data_ptr<int>() : nullptr),
                  "attention_tc");
+}
+
+// How the tiles of a step's tcgen05 attention are cut into pieces (attention_tc.cu): [pieces, 8] int32 in the order in which they start,
+// or an empty tensor where whole tiles are as good.  `seqs`: (tokens cached before the step, new tokens) of every sequence from `first_seq`
+// on.  Times are counted in blocks of 128 keys (about 0.9 us at head size 64): a CTA costs its blocks and kFixed more, a piece kMerge on top; the
+// CTAs go to the SM that is free first, longest first.  Whole tiles stay where they come within a tenth of the even share; otherwise every
+// tile is cut into equal pieces of at most P blocks, with the P of a few that ends first.
+Tensor attention_pieces(const std::vector<std::pair<int64_t, int64_t>>& seqs, int64_t first_seq, int64_t tokens_per_tile, int64_t kv_heads,
+                        int64_t window, int64_t chunk, int64_t sms) {
+    constexpr double kFixed = 7.0, kMerge = 6.0;
+    struct Tile { int seq, tok0, blocks; };
+    std::vector<Tile> tiles;
+    double total = 0;
+    for (size_t i = 0; i < seqs.size(); ++i)
+        for (int64_t t = 0; t < seqs[i].second; t += tokens_per_tile) {
+            const int64_t lo_pos = seqs[i].first + t, hi_pos = seqs[i].first + std::min(t + tokens_per_tile, seqs[i].second) - 1;
+            int64_t lo = window > 0 ? std::max<int64_t>(0, lo_pos - window + 1) : 0;
+            if (chunk > 0) lo = std::max(lo, lo_pos / chunk * chunk);
+            lo = lo / 128 * 128;
+            const int blocks = (int)((hi_pos + 1 - lo + 127) / 128);
+            tiles.push_back({(int)(first_seq + (int64_t)i), (int)t, blocks});
+            total += kv_heads * (blocks + kFixed);
+        }
+    std::stable_sort(tiles.begin(), tiles.end(), [](const Tile& a, const Tile& b) { return a.blocks > b.blocks; });
+    const Tensor none = torch::empty({0, 8}, torch::kInt32);
+    if (tiles.empty() || tiles[0].blocks < 8 || (double)tiles.size() * kv_heads > 16.0 * sms) return none;
+    // the time of cutting every tile into pieces of at most `most` blocks
+    auto ends_at = [&](int most) {
+        std::vector<double> costs;
+        for (const Tile& t : tiles) {
+            const int parts = (t.blocks + most - 1) / most;
+            const double cost = (double)t.blocks / parts + kFixed + (parts > 1 ? kMerge : 0.0);
+            costs.insert(costs.end(), (size_t)(parts * kv_heads), cost);
+        }
+        std::sort(costs.begin(), costs.end(), std::greater<double>());
+        std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+        double last = 0;
+        for (double c : costs) {
+            double at = c;
+            if ((int64_t)free_at.size() >= sms) {
+                at += free_at.top();
+                free_at.pop();
+            }
+            free_at.push(at);
+            last = std::max(last, at);
+        }
+        return last;
+    };
+    const double whole = ends_at(1 << 30), even = total / sms;
+    if (whole <= 1.1 * std::max(even, 24.0)) return none;
+    int best = 0;
+    double best_end = 0.95 * whole;
+    for (double part : {1.0, 0.75, 0.5, 0.38, 0.3, 0.22, 0.155}) {
+        const int most = std::max(8, (int)(even * part));
+        const double end = ends_at(most);
+        if (end < best_end) {
+            best_end = end;
+            best = most;
+        }
+    }
+    if (best == 0) return none;
+    struct Piece { int v[8]; };
+    std::vector<Piece> pieces;
+    for (size_t i = 0; i < tiles.size(); ++i) {
+        const Tile& t = tiles[i];
+        const int parts = (t.blocks + best - 1) / best;
+        for (int h = 0; h < kv_heads; ++h)
+            for (int q = 0; q < parts; ++q) {
+                const int a = (int)((int64_t)t.blocks * q / parts), b = (int)((int64_t)t.blocks * (q + 1) / parts);
+                pieces.push_back({{t.seq, t.tok0, h, (int)(i * kv_heads) + h, a, b - a, q, parts}});
+            }
+    }
+    Tensor out = torch::empty({(int64_t)pieces.size(), 8}, torch::kInt32);
+    std::memcpy(out.data_ptr<int>(), pieces.data(), pieces.size() * sizeof(Piece));
+    return out;
 }
 
 void attention_decode(const Tensor& qkv, Tensor& out, const Tensor& k_cache, const Tensor& v_cache, const Tensor& cu_q,
@@ -1601,10 +1695,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("n_splits"), py::arg("part_o") = py::none(), py::arg("part_ml") = py::none(),
           py::arg("status") = py::none(), py::arg("chunk") = 0, py::arg("sinks") = py::none(), py::arg("softcap") = 0.0);
     m.def("attention_tc_supports", &attention_tc_supports);
+    m.def("attention_pieces", &attention_pieces);
     m.def("attention_tc", &attention_tc, py::arg("qkv"), py::arg("out"), py::arg("k_cache"), py::arg("v_cache"),
           py::arg("cu_q"), py::arg("q_start"), py::arg("block_table"), py::arg("tiles"), py::arg("heads"),
           py::arg("kv_heads"), py::arg("head_dim"), py::arg("window"), py::arg("scale"), py::arg("status") = py::none(),
-          py::arg("chunk") = 0, py::arg("sinks") = py::none(), py::arg("softcap") = 0.0);
+          py::arg("chunk") = 0, py::arg("sinks") = py::none(), py::arg("softcap") = 0.0, py::arg("pieces") = py::none(), py::arg("part_o") = py::none(),
+          py::arg("part_ml") = py::none(), py::arg("counters") = py::none());
     m.def("attention_decode", &attention_decode, py::arg("qkv"), py::arg("out"), py::arg("k_cache"), py::arg("v_cache"),
           py::arg("cu_q"), py::arg("q_start"), py::arg("block_table"), py::arg("heads"), py::arg("kv_heads"),
           py::arg("head_dim"), py::arg("window"), py::arg("scale"), py::arg("n_splits"), py::arg("part_o") = py::none(),

@@ -917,6 +917,28 @@ def _attention_tiles(ctx, tokens_per_tile: int, device, first_seq: int = 0):
     return tiles
 
 
+def _attention_pieces(ctx, first_seq: int, tokens_per_tile: int, kv_heads: int, head_dim: int, window: int, chunk: int, device) -> dict:
+    """The arguments with which the tcgen05 attention runs its tiles in pieces, or none where whole tiles are as good (decided once a
+    step; the scratch is a launch's own)."""
+    if torch.device(device).type != "cuda":
+        return {}
+    key = ("attention_pieces", first_seq, tokens_per_tile, kv_heads, window, chunk)
+    pieces = ctx.extras.get(key)
+    if pieces is None:
+        sms = _sm_counts.get(device)
+        if sms is None:
+            sms = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+        host = backend().attention_pieces([(s.start, s.length) for s in ctx.seqs[first_seq:]], first_seq, tokens_per_tile, kv_heads, window, chunk, sms)
+        # (the counters are the step's own: every launch leaves them zero)
+        pieces = ctx.extras[key] = (host.pin_memory().to(device, non_blocking=True),
+                                    torch.zeros(host.shape[0], dtype=torch.int32, device=device)) if host.shape[0] else ()
+    if not pieces:
+        return {}
+    n = pieces[0].shape[0]
+    return {"pieces": pieces[0], "part_o": torch.empty(n * 128 * head_dim, dtype=torch.float32, device=device),
+            "part_ml": torch.empty(n * 256, dtype=torch.float32, device=device), "counters": pieces[1]}
+
+
 MIXED_STEP_MIN_SINGLES = 2    # single tokens at the head of a mixed step from which they get a launch of their own
 
 
@@ -1025,7 +1047,8 @@ def paged_attention(qkv, out, k_cache, v_cache, ctx, block_table, heads: int, kv
             # sum there too; a cap bends a row's scores where they arrive from tensor memory)
             tiles = _attention_tiles(ctx, 128 // group, qkv.device)
             be.attention_tc(qkv, out, k_cache, v_cache, ctx.cu_q, ctx.q_start, block_table, tiles, heads, kv_heads, head_dim, w,
-                            float(scale), status, chunk=c, sinks=sinks, softcap=float(softcap) if softcap else 0.0)
+                            float(scale), status, chunk=c, sinks=sinks, softcap=float(softcap) if softcap else 0.0,
+                            **_attention_pieces(ctx, 0, 128 // group, kv_heads, head_dim, w, c, qkv.device))
             return out
         splits, part_o, part_ml = 1, None, None
         if ctx.max_q_len == 1:
@@ -1084,7 +1107,8 @@ def paged_attention(qkv, out, k_cache, v_cache, ctx, block_table, heads: int, kv
                 lead = 0
             tiles = _attention_tiles(ctx, 128 // group, qkv.device, first_seq=lead)
             be.attention_tc(qkv, out, k_cache, v_cache, ctx.cu_q, ctx.q_start, block_table, tiles, heads, kv_heads,
-                            head_dim, w, float(scale), status, chunk=c)
+                            head_dim, w, float(scale), status, chunk=c,
+                            **_attention_pieces(ctx, lead, 128 // group, kv_heads, head_dim, w, c, qkv.device))
             return out
         # mma.sync tiles of 128 rows (8 warps) where the portions are long enough to fill them, else of 64
         warps = 8 if ctx.max_q_len * group >= 128 and be.attention_mma_supports(head_dim, heads, kv_heads, 8) else 4
