@@ -555,11 +555,12 @@ def design_points(design: str, sizes, steps: int, warmup: int) -> int:
         for n in names:
             setattr(ops, n, wrap(n, saved[n]))
         graphs, runner.use_graphs = runner.use_graphs, False
+        fused, ops.FUSE_LAYER = ops.FUSE_LAYER, False        # (a layer's kernels one by one)
         try:
             runner.step(entries)
             torch.cuda.synchronize()
         finally:
-            runner.use_graphs = graphs
+            runner.use_graphs, ops.FUSE_LAYER = graphs, fused
             for n in names:
                 setattr(ops, n, saved[n])
         total = {}

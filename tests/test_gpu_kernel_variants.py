@@ -170,3 +170,23 @@ def test_attention_tiles_in_pieces_equal_whole_tiles(monkeypatch, heads, kv_head
     whole = run()
     assert status.tolist() == [0, 0]
     assert float((first - whole).abs().max()) <= 2.0 ** -7 * max(1.0, float(whole.abs().max()))
+
+
+# (two rows, the bounds of the unadded shares and of their small weights, a tile of 256 and beyond it; single tokens beside portions)
+@pytest.mark.parametrize("lens", [[2], [7, 1, 1], [64, 64], [65, 64, 1], [256, 1], [301, 5]])
+def test_dense_layers_from_native_code_give_the_same_bits(tmp_path_factory, monkeypatch, lens):
+    """The same kernels in the same order, so the same logits, for a first portion and one behind cached tokens."""
+    import scenarios
+    folder = helpers.make_folder("D", str(tmp_path_factory.mktemp("dense")))
+    vocab = helpers.vocab_of(folder)
+    prompts = [[(31 * i + 7 * r + 1) % vocab for i in range(n + 40)] for r, n in enumerate(lens)]
+    trace = helpers.Trace()
+    trace.add([(r, 0, n) for r, n in enumerate(lens)], prompts)
+    trace.add([(r, n, 40) for r, n in enumerate(lens)], prompts, end=range(len(lens)))
+    got = []
+    for fused in (True, False):
+        o = ops()
+        monkeypatch.setattr(o, "FUSE_LAYER", fused)
+        runner = scenarios.runner_for(folder, DEV, "bfloat16", num_pages=helpers.tokens_needed(trace, round_to=16) // 16, max_requests=len(lens))
+        got.append(helpers.run_trace_inproc(runner, trace))
+    assert got[0].keys() == got[1].keys() and all((got[0][s] == got[1][s]).all() for s in got[0])

@@ -179,6 +179,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     int4 piece = make_int4(0, 1 << 30, 0, 1);            // (first block, blocks, which of the tile's pieces, how many)
     int tile_id = 0;
     if constexpr (PIECES) {
+        pdl_wait();                                      // (the pieces were copied to the device in the middle of the step)
         const int4 at = p.pieces[2 * blockIdx.x];
         piece = p.pieces[2 * blockIdx.x + 1];
         tl = make_int2(at.x, at.y);

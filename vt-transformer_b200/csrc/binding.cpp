@@ -1573,6 +1573,47 @@ void sample(const Tensor& logits, const Tensor& temperature, const Tensor& top_k
                                     logits.size(1), stream_of(logits)), "sample");
 }
 
+// A pre-norm layer of plain attention and a gated feed-forward, in bfloat16, as two calls with its attention between them: the same
+// kernels in the same order as one by one (rmsnorm, gemm_tc, rope_store; then gemm_tc, rmsnorm, gemm_tc, gemm_tc).  A step of a few dozen
+// tokens waits for the host, which takes some ten microseconds a kernel from Python and three from here.
+Tensor to_stream(const Tensor& x, const Tensor& w, c10::optional<Tensor> bias, c10::optional<Tensor> status, c10::optional<Tensor> scratch,
+                 c10::optional<Tensor> counters, int64_t share_rows, int64_t small_bytes, c10::optional<Tensor> next_w, int64_t next_epilogue,
+                 int64_t next_bytes) {
+    const int64_t m = x.size(0), n = w.size(0), k = w.size(1);
+    if (m > 0 && m <= share_rows && !(m > 128 && 2 * n * k <= small_bytes)) {
+        Tensor shares = torch::empty({(int64_t)vtb::gemm_tc_shares(m, n, k), m, n}, x.options().dtype(torch::kFloat32));
+        gemm_tc(x, w, bias, shares, status, c10::nullopt, c10::nullopt, 2, next_w, next_epilogue, next_bytes);
+        return shares;
+    }
+    Tensor out = torch::empty({m, n}, x.options());
+    gemm_tc(x, w, bias, out, status, scratch, counters, 0, next_w, next_epilogue, next_bytes);
+    return out;
+}
+
+Tensor dense_layer_in(Tensor& x, c10::optional<Tensor> delta, const Tensor& norm_weight, double eps, const Tensor& w_qkv, c10::optional<Tensor> b_qkv,
+                      const Tensor& positions, c10::optional<Tensor> cos_sin, Tensor& k_cache, Tensor& v_cache, const Tensor& token_seq,
+                      const Tensor& block_table, int64_t heads, int64_t kv_heads, int64_t head_dim, bool store, c10::optional<Tensor> status,
+                      c10::optional<Tensor> scratch, c10::optional<Tensor> counters, const Tensor& w_o, int64_t next_bytes) {
+    Tensor h = torch::empty(x.sizes(), x.options().dtype(torch::kBFloat16));
+    rmsnorm(x, delta, norm_weight, eps, h, c10::nullopt, status, c10::nullopt, 0.0, 1.0, 1, 1.0, false);
+    Tensor qkv = torch::empty({x.size(0), w_qkv.size(0)}, h.options());
+    gemm_tc(h, w_qkv, b_qkv, qkv, status, scratch, counters, 0, w_o, 2, next_bytes);
+    rope_store(qkv, positions, cos_sin, k_cache, v_cache, token_seq, block_table, heads, kv_heads, head_dim, store, status);
+    return qkv;
+}
+
+Tensor dense_layer_out(const Tensor& o, const Tensor& w_o, c10::optional<Tensor> b_o, Tensor& x, const Tensor& norm_weight, double eps,
+                       const Tensor& w_gate_up, const Tensor& w_down, c10::optional<Tensor> status, c10::optional<Tensor> scratch,
+                       c10::optional<Tensor> counters, int64_t share_rows, int64_t small_bytes, c10::optional<Tensor> then_w, int64_t then_epilogue,
+                       int64_t next_bytes) {
+    Tensor delta = to_stream(o, w_o, b_o, status, scratch, counters, share_rows, small_bytes, w_gate_up, 1, next_bytes);
+    Tensor h = torch::empty(x.sizes(), o.options());
+    rmsnorm(x, delta, norm_weight, eps, h, c10::nullopt, status, c10::nullopt, 0.0, 1.0, 1, 1.0, false);
+    Tensor act = torch::empty({x.size(0), w_gate_up.size(0) / 2}, o.options());
+    gemm_tc(h, w_gate_up, c10::nullopt, act, status, scratch, counters, 1, w_down, 2, next_bytes);
+    return to_stream(act, w_down, c10::nullopt, status, scratch, counters, share_rows, small_bytes, then_w, then_epilogue, next_bytes);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -1677,6 +1718,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("rope_store", &rope_store, py::arg("qkv"), py::arg("positions"), py::arg("cos_sin"), py::arg("k_cache"),
           py::arg("v_cache"), py::arg("token_seq"), py::arg("block_table"), py::arg("heads"), py::arg("kv_heads"),
           py::arg("head_dim"), py::arg("store"), py::arg("status") = py::none());
+    m.def("dense_layer_in", &dense_layer_in);
+    m.def("dense_layer_out", &dense_layer_out);
     m.def("gemm_simt", &gemm_simt, py::arg("a"), py::arg("w"), py::arg("bias"), py::arg("c"));
     m.def("attention_simt", &attention_simt, py::arg("qkv"), py::arg("out"), py::arg("k_cache"), py::arg("v_cache"),
           py::arg("positions"), py::arg("token_seq"), py::arg("block_table"), py::arg("heads"), py::arg("kv_heads"),

@@ -997,6 +997,34 @@ def rope_attention(qkv, out, cos_sin, k_cache, v_cache, ctx, block_table, heads:
                            status=status)
 
 
+FUSE_LAYER = True   # False: a dense layer's kernels are always called one by one (measurements of single kernels)
+
+
+def dense_layer_in(x, delta, norm_weight, eps: float, w_qkv, b_qkv, table, cache, ctx, w_o, heads: int, kv_heads: int, head_dim: int) -> torch.Tensor:
+    """What a pre-norm layer does before its attention, as one call: x += delta and its norm (``rmsnorm``), q, k and v (``linear``), their
+    rotation and the cache store (``rope_store``).  Returns q, k and v."""
+    global launches
+    launches += 3
+    scratch, counters = _split_workspace(x.device)
+    if isinstance(delta, SplitSum):
+        delta = delta.shares
+    return backend().dense_layer_in(x, delta, norm_weight, float(eps), w_qkv, b_qkv, ctx.positions, table, cache.k, cache.v, ctx.token_seq,
+                                    cache.block_table, heads, kv_heads, head_dim, bool(cache.writes), ctx.status, scratch, counters, w_o,
+                                    LOOK_AHEAD_BYTES)
+
+
+def dense_layer_out(o, w_o, b_o, x, norm_weight, eps: float, w_gate_up, w_down, status, then):
+    """What it does behind its attention: the o projection (``linear_to_stream``), the second norm with the sum, the gated feed-forward
+    (``linear_silu_mul``, ``linear_to_stream``).  Returns what the next norm adds, as ``linear_to_stream`` does."""
+    global launches
+    launches += 4
+    scratch, counters = _split_workspace(x.device)
+    then_w, then_epilogue = then if then is not None else (None, 0)
+    out = backend().dense_layer_out(o, w_o, b_o, x, norm_weight, float(eps), w_gate_up, w_down, status, scratch, counters,
+                                    STREAM_MAX_ROWS if STREAM_SHARES else 0, STREAM_SMALL_WEIGHT_BYTES, then_w, then_epilogue, LOOK_AHEAD_BYTES)
+    return SplitSum(out) if out.dim() == 3 else out
+
+
 FUSE_ROPE = True    # False: always the separate rotation kernel (tests compare the two)
 
 

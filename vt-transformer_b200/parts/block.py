@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import Block, ParamSpec, StateSpec, build_part, register_part
+from .base import Block, ParamSpec, ResidualStream, StateSpec, build_part, register_part
 
 
 @register_part("block", "prenorm")
@@ -11,6 +11,8 @@ class PreNormBlock(Block):
     """x += mixer(norm1(x)); x += ffn(norm2(x))
     (the order of v1/models/qwen2-7b/inference_fp16.dag:287-345).  The two sums are formed
     in 32-bit inside the next norm (``ResidualStream``)."""
+
+    dense = None            # whether the layer takes the native path; decided at the first step after its weights were loaded
 
     def __init__(self, spec, prefix, rt):
         super().__init__(spec, prefix, rt)
@@ -36,6 +38,7 @@ class PreNormBlock(Block):
         return out
 
     def load(self, get) -> None:
+        self.dense = None
         for p in self.parts:
             p.load(get)
 
@@ -52,7 +55,35 @@ class PreNormBlock(Block):
         self.mixer.then = self.ffn.first_product()
         self.ffn.then = then
 
+    def _dense(self) -> bool:
+        """Whether the layer is the plain dense one in bfloat16 throughout, whose kernels ``ops.dense_layer_in`` and ``dense_layer_out``
+        launch from native code."""
+        from .attention import PagedAttention
+        from .mlp import GatedMLP
+        from .norm import RMSNorm
+        if not (type(self) is PreNormBlock and type(self.norm1) is RMSNorm and type(self.norm2) is RMSNorm and type(self.mixer) is PagedAttention
+                and type(self.ffn) is GatedMLP and self.norm1.spec.groups == self.norm2.spec.groups == 1 and self.rt.dtype == torch.bfloat16):
+            return False
+        return all(w.dtype == torch.bfloat16 and w.is_contiguous() for w in (self.mixer.w_qkv, self.mixer.w_o, self.ffn.w_gate_up, self.ffn.w_down))
+
+    def _forward_dense(self, stream, ctx, cache) -> None:
+        ops, m, f, s = self.rt.ops, self.mixer, self.ffn, self.mixer.spec
+        delta, stream.pending = stream.pending, None
+        qkv = ops.dense_layer_in(stream.x, delta, self.norm1.weight, self.norm1.spec.eps, m.w_qkv, m.b_qkv, m.position.table, cache, ctx, m.w_o,
+                                 s.heads, s.kv_heads, s.head_dim)
+        o = torch.empty((qkv.shape[0], m.q_dim), dtype=qkv.dtype, device=qkv.device)
+        ops.paged_attention(qkv, o, cache.k, cache.v, ctx, cache.block_table, s.heads, s.kv_heads, s.head_dim, s.window, m.scale, status=ctx.status)
+        stream.add(ops.dense_layer_out(o, m.w_o, m.b_o, stream.x, self.norm2.weight, self.norm2.spec.eps, f.w_gate_up, f.w_down, ctx.status, f.then))
+
     def forward(self, stream, ctx, cache):
+        ops = self.rt.ops
+        if self.dense is None:
+            self.dense = self._dense()
+        if (self.dense and stream.x.is_cuda and type(stream) is ResidualStream and stream.pending_post is None and ops.FUSE_LAYER and ops.FUSE_SILU
+                and ops.SMALL_BATCH_KERNEL == "tc" and not ops.single_token_step_is_one_kernel(
+                    ctx, self.rt.dtype, self.mixer.spec.heads, self.mixer.spec.kv_heads, self.mixer.spec.head_dim)):
+            self._forward_dense(stream, ctx, cache)
+            return
         h = stream.normed(self.norm1)
         stream.add(self.mixer.forward(h, ctx, cache))
         if self.ffn is None:
