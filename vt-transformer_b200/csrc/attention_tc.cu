@@ -27,7 +27,8 @@
 // A tile's blocks may be cut into pieces, a CTA each, where whole tiles would leave SMs idle (few tiles over long contexts, a last round
 // that is nearly empty; the caller decides, see attention_pieces in binding.cpp).  A piece leaves its rows' unnormalised results with
 // their maxima and sums in scratch memory, and the CTA of a tile that arrives last (a counter a tile, left zero) puts the pieces
-// together in their order; no CTA waits for another.
+// together in their order; no CTA waits for another.  Measured on a B200: 2,048 tokens behind 30,720 (14 heads over 2 of 64), the whole step
+// 14.25 ms with whole tiles (228 of them on 148 SMs), 13.26 in pieces; the kernel of whole tiles is compiled apart, since the pieces' code slowed it.
 //
 // Warp 0 loads (one thread), warp 1 issues the MMAs (one thread), warps 2..5 and 6..9 are the two groups.
 // Every wait on a barrier is bounded; a wait that runs out sets the status word and the CTA winds down.
